@@ -540,10 +540,10 @@ int ob_probe_fp64(double *dfma_lane_per_s);
  * look-back wait of the Morton ordering; no reference counterpart. */
 int ob_test_lookback_timeout(uint64_t n, uint32_t poll_limit, int skip_first_tile);
 
-/* Bounds the FP32 tree walk's per-warp traversal stack of `solver` to `cap`
- * entries (0 restores the full 256) from its next evaluation on. A warp whose
- * stack fills discards its partial sums and finishes with the per-target
- * union walk (the fallback a valid tree rarely needs); a small cap forces it,
+/* Bounds the FP32 tree walk's traversal stack of `solver` to `cap` (at most
+ * 256) entries (0 restores the full stack) from its next evaluation on. A group
+ * of targets whose stack fills discards its partial sums and finishes with the
+ * per-target union walk (the fallback a valid tree rarely needs); a small cap forces it,
  * so tests can hold that path to the oracle. OB_ERROR_UNSUPPORTED for direct
  * or FP64 solvers. No reference counterpart. */
 int ob_test_set_walk_stack_cap(ob_solver *solver, uint32_t cap);

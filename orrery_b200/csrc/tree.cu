@@ -195,7 +195,7 @@ __global__ void __launch_bounds__(kThreads)
 __global__ void __launch_bounds__(kThreads)
     layout_write_kernel(const unsigned long long *__restrict__ codes, uint32_t n, uint32_t cap,
                         const uint32_t *__restrict__ offsets, uint32_t capacity,
-                        DeviceNode *nodes, uint32_t *children, uint32_t *child_slots,
+                        DeviceNode *nodes, uint32_t *child_mask, uint32_t *child_slots,
                         TreeMeta *meta, unsigned *status) {
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         const uint32_t total = offsets[n];
@@ -243,17 +243,11 @@ __global__ void __launch_bounds__(kThreads)
             node.first = b;
             node.level = level;
             node.parent = parent;
-            node.pad = 0;
+            node.octant = level == 0 ? 0u : static_cast<uint32_t>(prefix(codes[b], level) & 7u);
             nodes[index] = node;
             if (parent != index) {
-                // A cell has at most eight children; their slots are filled
-                // in arrival order and sorted by the moments pass.
-                const uint32_t slot = atomicAdd(&children[parent], 1u);
-                if (slot < kMaxChildren) {
-                    child_slots[static_cast<size_t>(parent) * kMaxChildren + slot] = index;
-                } else {
-                    atomicOr(status, kStatusInvalid);
-                }
+                atomicOr(&child_mask[parent], 1u << node.octant);
+                child_slots[static_cast<size_t>(parent) * kMaxChildren + node.octant] = index;
             }
             parent = index;
             if (leaf) {
@@ -326,54 +320,48 @@ __device__ double acceptance(const TreeMeta *meta, unsigned long long code, uint
     return __dmul_rn(radius, radius);
 }
 
-// Sorts eight values in registers (Batcher's odd-even merge network).
-__device__ __forceinline__ void sort8(uint32_t (&v)[8]) {
-    constexpr int kPairs[19][2] = {{0, 1}, {2, 3}, {4, 5}, {6, 7}, {0, 2}, {1, 3}, {4, 6},
-                                   {5, 7}, {1, 2}, {5, 6}, {0, 4}, {1, 5}, {2, 6}, {3, 7},
-                                   {2, 4}, {3, 5}, {1, 2}, {3, 4}, {5, 6}};
-#pragma unroll
-    for (int p = 0; p < 19; ++p) {
-        const uint32_t a = v[kPairs[p][0]], b = v[kPairs[p][1]];
-        v[kPairs[p][0]] = min(a, b);
-        v[kPairs[p][1]] = max(a, b);
+// Writes the walk's compact record of a node at its slot (see WalkNodes): a
+// leaf's link is its first particle, an internal node's the slot of its first
+// child.
+__device__ void store_walk_node(const WalkNodes &walk, uint32_t slot, uint32_t k, double cx,
+                                double cy, double cz, double mass, double r2,
+                                const DeviceQuadrupole *q, uint32_t link, uint32_t word) {
+    const float hx = __double2float_rn(cx);
+    const float hy = __double2float_rn(cy);
+    const float hz = __double2float_rn(cz);
+    walk.a[slot] = make_float4(hx, hy, hz, __double2float_rn(mass));
+    walk.b[slot] = make_float4(__double2float_rn(__dsub_rn(cx, static_cast<double>(hx))),
+                               __double2float_rn(__dsub_rn(cy, static_cast<double>(hy))),
+                               __double2float_rn(__dsub_rn(cz, static_cast<double>(hz))),
+                               __double2float_rn(r2));
+    float4 d = make_float4(0.0f, 0.0f, __uint_as_float(link), __uint_as_float(word));
+    if (q != nullptr) {
+        walk.c[slot] = make_float4(__double2float_rn(q->xx), __double2float_rn(q->xy),
+                                   __double2float_rn(q->xz), __double2float_rn(q->yy));
+        d.x = __double2float_rn(q->yz);
+        d.y = __double2float_rn(q->zz);
     }
+    walk.d[slot] = d;
+    walk.node[slot] = k;
 }
 
-// Writes the walk's compact record of node k (see WalkNode). `sibling`: the
-// node has a next sibling, i.e. its escape index lies inside its parent's
-// subtree (carried in the top bit of the count word). A leaf's escape index is
-// always k + 1, so a leaf's record carries its first particle in its place.
-__device__ void store_walk_node(WalkNode *walk, uint32_t *first_of, uint32_t k,
-                                const DeviceNode &node, const DeviceQuadrupole *q,
-                                bool sibling) {
-    const uint32_t count_word = node.count | (sibling ? kWalkSiblingBit : 0u);
-    const uint32_t link = node.count > 0 ? node.first : node.next;
-    const float hx = __double2float_rn(node.com_x);
-    const float hy = __double2float_rn(node.com_y);
-    const float hz = __double2float_rn(node.com_z);
-    WalkNode w;
-    w.a = make_float4(hx, hy, hz, __double2float_rn(node.mass));
-    w.b = make_float4(__double2float_rn(__dsub_rn(node.com_x, static_cast<double>(hx))),
-                      __double2float_rn(__dsub_rn(node.com_y, static_cast<double>(hy))),
-                      __double2float_rn(__dsub_rn(node.com_z, static_cast<double>(hz))),
-                      __double2float_rn(node.r2));
-    if (q != nullptr) {
-        w.c = make_float4(__double2float_rn(q->xx), __double2float_rn(q->xy),
-                          __double2float_rn(q->xz), __double2float_rn(q->yy));
-        w.d = make_float4(__double2float_rn(q->yz), __double2float_rn(q->zz),
-                          __uint_as_float(link), __uint_as_float(count_word));
-    } else {
-        w.c = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        w.d = make_float4(0.0f, 0.0f, __uint_as_float(link), __uint_as_float(count_word));
-    }
-    walk[k] = w;
-    first_of[k] = node.first;
+// Right siblings of a child in `octant` of a cell with these children.
+__device__ __forceinline__ uint32_t right_siblings(uint32_t mask, uint32_t octant) {
+    return static_cast<uint32_t>(__popc(mask >> (octant + 1u)));
+}
+
+// The slot of the child in `octant` of `parent` (whose children are `mask`):
+// 1 + parent + P(parent) + its left siblings, with right = P(child).
+__device__ __forceinline__ uint32_t slot_of(uint32_t parent, uint32_t right, uint32_t mask,
+                                            uint32_t octant) {
+    return 1u + parent + (right - right_siblings(mask, octant)) +
+           static_cast<uint32_t>(__popc(mask & ((1u << octant) - 1u)));
 }
 
 __global__ void __launch_bounds__(kThreads)
     moments_kernel(const double *__restrict__ sorted, const unsigned long long *__restrict__ codes,
-                   uint32_t n, DeviceNode *nodes, DeviceQuadrupole *quads, WalkNode *walk,
-                   uint32_t *first_of, const uint32_t *__restrict__ children,
+                   uint32_t n, DeviceNode *nodes, DeviceQuadrupole *quads, WalkNodes walk,
+                   const uint32_t *__restrict__ child_mask,
                    const uint32_t *__restrict__ child_slots, uint32_t *arrived,
                    float4 *leaf_rel, TreeMeta *meta, double theta) {
     const double *X = sorted;
@@ -420,50 +408,62 @@ __global__ void __launch_bounds__(kThreads)
                                       __double2float_rn(__dsub_rn(Z[i], cz)),
                                       __double2float_rn(M[i]));
         }
+        // Slots: the children of node j (pre-order index) start at slot
+        // 1 + j + P(j), where P(j) sums the right siblings of j and of each of
+        // its ancestors: the nodes before j and these siblings are exactly
+        // those whose parents come before j. `right` is P of the node at hand.
+        uint32_t right = 0;
+        for (uint32_t a = k, climb = 0; climb < 64u; ++climb) {
+            const uint32_t up = nodes[a].parent;
+            if (up == a) {
+                break;
+            }
+            right += right_siblings(child_mask[up], nodes[a].octant);
+            a = up;
+        }
+
         const uint32_t level = nodes[k].level;
+        const double r2 = acceptance(meta, codes[begin], level, cx, cy, cz, theta);
         nodes[k].mass = mass;
         nodes[k].com_x = cx;
         nodes[k].com_y = cy;
         nodes[k].com_z = cz;
-        nodes[k].r2 = acceptance(meta, codes[begin], level, cx, cy, cz, theta);
+        nodes[k].r2 = r2;
         if (with_quads) {
             quads[k] = q;
         }
-        {
-            // Escape indices and parents were written by the layout kernel.
-            const uint32_t up = nodes[k].parent;
-            const bool sibling = up != k && nodes[k].next < nodes[up].next;
-            store_walk_node(walk, first_of, k, nodes[k], with_quads ? &q : nullptr, sibling);
-        }
-
         // Climb while this thread completes its parent (gather_moments,
         // octree.cpp:142-185). A cell has at most 22 ancestors.
         uint32_t current = k;
+        uint32_t parent = nodes[k].parent;
+        uint32_t octant = nodes[k].octant;
+        uint32_t mask = parent == current ? 0u : child_mask[parent];
+        {
+            const uint32_t slot = parent == current ? 0u : slot_of(parent, right, mask, octant);
+            store_walk_node(walk, slot, k, cx, cy, cz, mass, r2, with_quads ? &q : nullptr,
+                            begin, kWalkLeafBit | (end - begin));
+        }
         for (int climb = 0; climb < 64; ++climb) {
-            __threadfence();
-            const uint32_t parent = nodes[current].parent;
             if (parent == current) {
                 break;
             }
+            __threadfence();
             const uint32_t before = atomicAdd(&arrived[parent], 1u);
-            if (before + 1 != children[parent]) {
+            const uint32_t kids = static_cast<uint32_t>(__popc(mask));
+            if (before + 1 != kids) {
                 break;
             }
             __threadfence();
-            const uint32_t stop = __ldcg(&nodes[parent].next);
-            // The parent's children in index (octant) order: its slots,
-            // sorted, so that their loads need no walk along escape indices.
-            const uint32_t kids = min(children[parent], kMaxChildren);
+            // The parent's children by octant, loaded at once.
             const uint4 *slots =
                 reinterpret_cast<const uint4 *>(child_slots + static_cast<size_t>(parent) *
                                                                   kMaxChildren);
             const uint4 s0 = __ldcg(slots), s1 = __ldcg(slots + 1);
             uint32_t kid[kMaxChildren] = {s0.x, s0.y, s0.z, s0.w, s1.x, s1.y, s1.z, s1.w};
 #pragma unroll
-            for (uint32_t k = 0; k < kMaxChildren; ++k) {
-                kid[k] = k < kids && kid[k] < count_nodes ? kid[k] : 0xffffffffu;
+            for (uint32_t o = 0; o < kMaxChildren; ++o) {
+                kid[o] = ((mask >> o) & 1u) != 0u && kid[o] < count_nodes ? kid[o] : 0xffffffffu;
             }
-            sort8(kid);
             double pm = 0.0, px = 0.0, py = 0.0, pz = 0.0, mx = 0.0, my = 0.0, mz = 0.0;
 #pragma unroll
             for (uint32_t k = 0; k < kMaxChildren; ++k) {
@@ -493,8 +493,8 @@ __global__ void __launch_bounds__(kThreads)
                 gy = __ddiv_rn(my, cnt);
                 gz = __ddiv_rn(mz, cnt);
             }
+            DeviceQuadrupole moment{0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
             if (with_quads) {
-                DeviceQuadrupole moment{0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
 #pragma unroll
                 for (uint32_t k = 0; k < kMaxChildren; ++k) {
                     if (kid[k] != 0xffffffffu) {
@@ -513,29 +513,23 @@ __global__ void __launch_bounds__(kThreads)
                 }
                 quads[parent] = moment;
             }
-            const uint32_t plevel = __ldcg(&nodes[parent].level);
-            const uint32_t pfirst = __ldcg(&nodes[parent].first);
+            const uint32_t plevel = nodes[parent].level;
+            const uint32_t pfirst = nodes[parent].first;
+            const double pr2 = acceptance(meta, codes[pfirst], plevel, gx, gy, gz, theta);
             nodes[parent].mass = pm;
             nodes[parent].com_x = gx;
             nodes[parent].com_y = gy;
             nodes[parent].com_z = gz;
-            nodes[parent].r2 = acceptance(meta, codes[pfirst], plevel, gx, gy, gz, theta);
-            {
-                DeviceNode copy;
-                copy.com_x = gx;
-                copy.com_y = gy;
-                copy.com_z = gz;
-                copy.mass = pm;
-                copy.r2 = nodes[parent].r2;
-                copy.next = stop;
-                copy.count = 0;
-                copy.first = pfirst;
-                const DeviceQuadrupole *pq = with_quads ? &quads[parent] : nullptr;
-                const uint32_t up = __ldcg(&nodes[parent].parent);
-                const bool sibling = up != parent && stop < __ldcg(&nodes[up].next);
-                store_walk_node(walk, first_of, parent, copy, pq, sibling);
-            }
+            nodes[parent].r2 = pr2;
+            right -= right_siblings(mask, octant); // now P(parent)
+            const uint32_t link = 1u + parent + right;
             current = parent;
+            parent = nodes[current].parent;
+            octant = nodes[current].octant;
+            mask = parent == current ? 0u : child_mask[parent];
+            const uint32_t slot = parent == current ? 0u : slot_of(parent, right, mask, octant);
+            store_walk_node(walk, slot, current, gx, gy, gz, pm, pr2,
+                            with_quads ? &moment : nullptr, link, kids);
         }
     }
 }
@@ -552,26 +546,26 @@ cudaError_t launch_layout_count(const unsigned long long *codes, uint32_t n, uin
 
 cudaError_t launch_layout_write(const unsigned long long *codes, uint32_t n, uint32_t leaf_cap,
                                 const uint32_t *offsets, uint32_t node_capacity,
-                                DeviceNode *nodes, uint32_t *children, uint32_t *child_slots,
+                                DeviceNode *nodes, uint32_t *child_mask, uint32_t *child_slots,
                                 TreeMeta *meta, unsigned *status, cudaStream_t stream) {
     layout_write_kernel<<<grid_for(n), kThreads, 0, stream>>>(codes, n, leaf_cap, offsets,
-                                                             node_capacity, nodes, children,
+                                                             node_capacity, nodes, child_mask,
                                                              child_slots, meta, status);
     return cudaGetLastError();
 }
 
 cudaError_t launch_moments(const double *sorted, const unsigned long long *codes, uint32_t n,
-                           DeviceNode *nodes, DeviceQuadrupole *quads, WalkNode *walk_nodes,
-                           uint32_t *first_of, const uint32_t *children,
-                           const uint32_t *child_slots, uint32_t *arrived, float4 *leaf_rel,
+                           DeviceNode *nodes, DeviceQuadrupole *quads, const WalkNodes &walk,
+                           const uint32_t *child_mask, const uint32_t *child_slots,
+                           uint32_t *arrived, float4 *leaf_rel,
                            TreeMeta *meta, double opening_angle, uint32_t node_capacity,
                            cudaStream_t stream) {
     if (reinterpret_cast<uintptr_t>(child_slots) % 16u != 0u) {
         return cudaErrorMisalignedAddress; // the climb reads a node's slots as two uint4
     }
     moments_kernel<<<grid_for(node_capacity), kThreads, 0, stream>>>(
-        sorted, codes, n, nodes, quads, walk_nodes, first_of, children, child_slots, arrived,
-        leaf_rel, meta, opening_angle);
+        sorted, codes, n, nodes, quads, walk, child_mask, child_slots, arrived, leaf_rel, meta,
+        opening_angle);
     return cudaGetLastError();
 }
 
@@ -625,11 +619,11 @@ void TreePipeline::reserve(uint32_t n) {
         if (params_.quadrupole) {
             quads_.reserve(want);
         }
-        walk_nodes_.reserve(want);
-        first_of_.reserve(want);
+        walk_records_.reserve(4ull * want);
+        walk_index_.reserve(want);
         // kMaxChildren child slots per node (first, so that a node's slots
         // start on a 16-byte boundary for their vector loads), then child
-        // counts and arrival counts.
+        // masks and arrival counts.
         level_lists_.reserve((kMaxChildren + 2ull) * want);
         node_capacity_ = want;
     }
@@ -658,7 +652,7 @@ void TreePipeline::evaluate(uint32_t n, const double *x, const double *y, const 
           "clearing tile tickets");
     check(cudaMemsetAsync(level_lists_.data() + kMaxChildren * static_cast<size_t>(node_capacity_),
                           0, sizeof(uint32_t) * 2ull * node_capacity_, stream),
-          "clearing child counts");
+          "clearing child masks");
 
     // Ordering: cube, codes + histograms, eight onesweep passes, gather.
     check(launch_bounding_cube(x, y, z, n, reduce_.data(), meta_.data(), stream), "cube");
@@ -688,15 +682,18 @@ void TreePipeline::evaluate(uint32_t n, const double *x, const double *y, const 
     check(launch_layout_count(codes, n, cap, counts, stream), "node counts");
     check(launch_exclusive_scan(counts, offsets, n, scan_partials_.data(), stream), "node scan");
     uint32_t *child_slots = level_lists_.data();
-    uint32_t *children = child_slots + kMaxChildren * static_cast<size_t>(node_capacity_);
-    uint32_t *arrived = children + node_capacity_;
-    check(launch_layout_write(codes, n, cap, offsets, node_capacity_, nodes_.data(), children,
+    uint32_t *child_mask = child_slots + kMaxChildren * static_cast<size_t>(node_capacity_);
+    uint32_t *arrived = child_mask + node_capacity_;
+    float4 *records = walk_records_.data();
+    const WalkNodes walk{records, records + node_capacity_, records + 2ull * node_capacity_,
+                         records + 3ull * node_capacity_, walk_index_.data()};
+    check(launch_layout_write(codes, n, cap, offsets, node_capacity_, nodes_.data(), child_mask,
                               child_slots, meta_.data(), status, stream),
           "node layout");
     check(launch_moments(sorted_.data(), codes, n, nodes_.data(),
-                         params_.quadrupole ? quads_.data() : nullptr, walk_nodes_.data(),
-                         first_of_.data(), children, child_slots, arrived, leaf_rel_.data(),
-                         meta_.data(), params_.opening_angle, node_capacity_, stream),
+                         params_.quadrupole ? quads_.data() : nullptr, walk, child_mask,
+                         child_slots, arrived, leaf_rel_.data(), meta_.data(),
+                         params_.opening_angle, node_capacity_, stream),
           "moments");
     record(built, stream, external);
 
@@ -708,10 +705,9 @@ void TreePipeline::evaluate(uint32_t n, const double *x, const double *y, const 
               "FP64 tree walk");
         return;
     }
-    check(launch_walk(nodes_.data(), walk_nodes_.data(), first_of_.data(), leaf_rel_.data(),
-                      sorted_.data(), perm, n, params_.softening_squared,
-                      params_.quadrupole != 0, ax, ay, az, meta_.data(), counters_.data(),
-                      status, stream, walk_stack_cap_),
+    check(launch_walk(nodes_.data(), params_.quadrupole ? quads_.data() : nullptr, walk,
+                      leaf_rel_.data(), sorted_.data(), perm, n, params_.softening_squared, ax,
+                      ay, az, meta_.data(), counters_.data(), status, stream, walk_stack_cap_),
           "tree walk");
 }
 

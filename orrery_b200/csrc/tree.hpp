@@ -26,31 +26,32 @@ struct alignas(16) DeviceNode {
     uint32_t first;      // first particle of the cell (sorted order)
     uint32_t level;      // depth of the cell (root 0)
     uint32_t parent;     // parent node (the root points at itself)
-    uint32_t pad;
+    uint32_t octant;     // the octant of its parent that the cell fills
 };
 static_assert(sizeof(DeviceNode) == 64, "DeviceNode is four 16-byte words");
 
-// The walk's compact copy of a node, four 16-byte words:
+// The walk's compact copies of the nodes, four 16-byte words each, one array
+// per word:
 //   a = (com_x hi, com_y hi, com_z hi, mass)       FP32
 //   b = (com_x lo, com_y lo, com_z lo, r2)         FP32 (r2 rounded to nearest)
 //   c = (Qxx, Qxy, Qxz, Qyy)                       FP32 quadrupole
-//   d = (Qyz, Qzz, link, count)                    link/count as uint32 bits:
-//                                                   link is the escape index of
-//                                                   an internal node and the
-//                                                   first particle of a leaf
-//                                                   (whose escape index is its
-//                                                   own + 1); the top bit of
-//                                                   count is set when the node
-//                                                   has a next sibling (escape
-//                                                   index < parent's)
+//   d = (Qyz, Qzz, link, word)                     link/word as uint32 bits: of
+//                                                   an internal node the slot
+//                                                   of its first child and its
+//                                                   number of children; of a
+//                                                   leaf its first particle and
+//                                                   kWalkLeafBit | its count
 // hi + lo carries each FP64 coordinate to ~2^-48 relative, so offsets to the
 // target (also split) come out in FP32 to ~1e-7 relative without conversions.
-struct alignas(16) WalkNode {
-    float4 a, b, c, d;
+// The children of a node fill consecutive slots (the root is slot 0), so the
+// walk reads a whole family with one 128-byte line per word where the
+// pre-order copies of eight siblings lay in up to eight lines; `node` gives a
+// slot's node in pre-order.
+struct WalkNodes {
+    float4 *a, *b, *c, *d;
+    uint32_t *node;
 };
-constexpr uint32_t kWalkSiblingBit = 0x80000000u;
-constexpr uint32_t kWalkCountMask = 0x7fffffffu;
-static_assert(sizeof(WalkNode) == 64, "WalkNode is four 16-byte words");
+constexpr uint32_t kWalkLeafBit = 0x80000000u;
 
 // Traceless quadrupole (include/orrery/solvers/octree.hpp:89-96).
 struct DeviceQuadrupole {
@@ -136,9 +137,9 @@ private:
     DeviceArray<uint32_t> scan_partials_;        // block sums of the scan
     DeviceArray<DeviceNode> nodes_;
     DeviceArray<DeviceQuadrupole> quads_;        // FP64 moments (parity, upward pass)
-    DeviceArray<WalkNode> walk_nodes_;           // compact FP32 node records the walk reads
-    DeviceArray<uint32_t> first_of_;             // first particle of each node (leaves)
-    DeviceArray<uint32_t> level_lists_;          // child slots, child counts, arrival counts
+    DeviceArray<float4> walk_records_;           // compact FP32 node records the walk reads
+    DeviceArray<uint32_t> walk_index_;           // the node of each walk record
+    DeviceArray<uint32_t> level_lists_;          // child slots, child masks, arrival counts
     DeviceArray<TreeMeta> meta_;
     DeviceArray<double> reduce_;                 // cube min/max partials
     DeviceArray<unsigned long long> counters_;   // pair and cell counts (accumulating)

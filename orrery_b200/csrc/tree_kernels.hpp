@@ -75,35 +75,36 @@ cudaError_t launch_exclusive_scan(const uint32_t *in, uint32_t *out, uint32_t n,
 cudaError_t launch_layout_count(const unsigned long long *codes, uint32_t n, uint32_t leaf_cap,
                                 uint32_t *counts, cudaStream_t stream);
 
-// Writes the node records (escape, first, count, level, parent), counts each
-// internal node's children and lists them (in arrival order) in its
-// kMaxChildren slots of child_slots. `offsets` is the exclusive scan of counts.
+// Writes the node records (escape, first, count, level, parent, octant), marks
+// each internal node's children by octant in child_mask (zeroed beforehand) and
+// lists them in its kMaxChildren child_slots, one per octant. `offsets` is the
+// exclusive scan of counts.
 constexpr uint32_t kMaxChildren = 8;
 cudaError_t launch_layout_write(const unsigned long long *codes, uint32_t n, uint32_t leaf_cap,
                                 const uint32_t *offsets, uint32_t node_capacity,
-                                DeviceNode *nodes, uint32_t *children, uint32_t *child_slots,
+                                DeviceNode *nodes, uint32_t *child_mask, uint32_t *child_slots,
                                 TreeMeta *meta, unsigned *status, cudaStream_t stream);
 
 // Moments bottom-up (mass, centre of mass, quadrupole, acceptance radius) and
 // the leaf-relative FP32 source positions the walk reads.
 cudaError_t launch_moments(const double *sorted, const unsigned long long *codes, uint32_t n,
-                           DeviceNode *nodes, DeviceQuadrupole *quads, WalkNode *walk_nodes,
-                           uint32_t *first_of, const uint32_t *children,
-                           const uint32_t *child_slots, uint32_t *arrived, float4 *leaf_rel,
+                           DeviceNode *nodes, DeviceQuadrupole *quads, const WalkNodes &walk,
+                           const uint32_t *child_mask, const uint32_t *child_slots,
+                           uint32_t *arrived, float4 *leaf_rel,
                            TreeMeta *meta, double opening_angle, uint32_t node_capacity,
                            cudaStream_t stream);
 
 // ------------------------------------------------------------------- walk
 
-// Accelerations written in the caller's (unsorted) order through perm;
-// pair and cell counts added to counters[0] and counters[1]. stack_cap (0 =
-// the walk's full per-warp stack) bounds the group traversal's stack; a warp
-// whose stack fills finishes with the per-target union walk.
+// Accelerations written in the caller's (unsorted) order through perm; pair
+// and cell counts added to counters[0] and counters[1]. `quads` NULL: monopoles
+// only. stack_cap (0 = the walk's full stack) bounds the group traversal's
+// stack; a group whose stack fills finishes with the per-target union walk.
 uint32_t walk_stack_capacity();
-cudaError_t launch_walk(const DeviceNode *nodes, const WalkNode *walk_nodes,
-                        const uint32_t *first_of, const float4 *leaf_rel, const double *sorted,
-                        const uint32_t *perm, uint32_t n, double eps2, bool quadrupole,
-                        double *ax, double *ay, double *az, TreeMeta *meta,
+cudaError_t launch_walk(const DeviceNode *nodes, const DeviceQuadrupole *quads,
+                        const WalkNodes &walk, const float4 *leaf_rel, const double *sorted,
+                        const uint32_t *perm, uint32_t n, double eps2, double *ax, double *ay,
+                        double *az, TreeMeta *meta,
                         unsigned long long *counters, unsigned *status, cudaStream_t stream,
                         uint32_t stack_cap = 0);
 

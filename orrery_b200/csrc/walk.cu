@@ -1,4 +1,5 @@
-// Barnes-Hut theta-criterion walk, one warp per 32 Morton-consecutive targets.
+// Barnes-Hut theta-criterion walk, one group of warps per 32 Morton-consecutive
+// targets.
 //
 // Semantics are those of walk_tree (src/solvers/tree_walk.cpp:20-83) for every
 // target separately: a cell is accepted when |com - x|^2 >= r2 in FP64 (the
@@ -8,13 +9,17 @@
 // a pair sum that skips the target itself; an opened internal node is
 // descended. Pair and cell counts are the reference's.
 //
-// Group traversal. The warp walks the tree once for its 32 targets, carrying
+// Group traversal. The group walks the tree once for its 32 targets, carrying
 // with every node the mask of targets whose own walks reach it (those that
-// opened all its ancestors). Lanes take different nodes of a depth-first
-// stack of (node, reach mask) items, up to 32 per round; an item pushes its
-// next sibling (a bit of the node record says whether it has one) and, when
-// opened, its first child. Each lane classifies its node against the
-// bounding box of the warp's targets from the node's compact record: the
+// opened all its ancestors). The depth-first stack holds families: the
+// children of one opened node, which fill consecutive slots of the walk's
+// records (tree.hpp), with the mask. A warp takes up to four families a round,
+// one child per lane, so eight lanes read 128 consecutive bytes of each record
+// word and a node's children are all met in the round after it. (With one
+// stack item per node that pushed its next sibling, a path down the tree cost
+// one round per sibling: 104 us for 1,000 particles, bound by that chain.)
+// Each lane classifies its node against the
+// bounding box of the group's targets from the node's compact record: the
 // per-axis distances from the centre of mass to the nearest and farthest box
 // faces are formed from FP32 hi + lo parts (so each is accurate to a few ulps
 // of itself), and with a 4e-6 relative margin on the acceptance radius
@@ -28,21 +33,31 @@
 // The lane that accepts a cell stages it at once in shared memory (centre of
 // mass relative to the box centre G, mass, 2.5 Q, target mask), packed so that
 // one 16-byte load gives two cells' values; an opened leaf is queued with its
-// centre relative to G, its particle range and mask. Batches of cells are then
-// evaluated by every lane for its own target, two cells per packed FP32x2
-// instruction (a lane outside a cell's mask contributes exactly zero), and
-// queued leaves likewise, their sources staged in shared memory per leaf.
+// centre, its particle range and mask. Batches of cells are then evaluated by
+// every lane for its own target, two cells per packed FP32x2 instruction (a
+// lane outside a cell's mask contributes exactly zero), and queued leaves
+// likewise, their sources staged in shared memory per leaf.
+//
+// Warps per group. A system of few groups leaves the GPU idle with one warp
+// each, so W warps (1, 2, 4 or 8, a CTA) share a group's traversal: every
+// round they take families round-robin off one stack, stage and evaluate what
+// they took for the same 32 targets, and push through counts exchanged at a
+// barrier; the W sums of a target are added in warp order, so results do not
+// depend on scheduling. launch_walk states where the lines lie.
 //
 // Arithmetic. Positions and centres of mass are carried as FP32 hi + lo pairs
 // (exact to ~2^-48 relative); force terms are FP32, summed in FP32 within a
-// batch and flushed into FP64 per-target sums.
+// batch (in blocks, so that chains stay short) and flushed into FP64 per-target
+// sums. A leaf's offset to the target is formed from hi and lo parts, so a
+// near source's distance does not carry the rounding of the box's size (a
+// 1,000-particle collision: relative force error 1.4e-7, against 5.0e-7 with
+// offsets through the box centre).
 //
-// A round takes no more items than the stack has room to push back (each
-// pushes at most two), so the stack (256 entries per warp; with this rule the
-// 2M two-disc collision rarely fills it) only stops the traversal when
-// completely full;
-// the warp then discards its partial sums and walks its targets with the
-// per-target union walk (union_walk below), which gives the same counts.
+// A round takes no more families than the stack has room to push back (eight
+// for each one taken), so the stack (256 entries per warp, at most 1024) only
+// stops the traversal when completely full; the group then discards its
+// partial sums and walks its targets with the per-target union walk
+// (union_walk below), which gives the same counts.
 //
 // Warp discipline. Between the warp's votes and barriers there is no long
 // lane-divergent stretch of work: lanes outside a leaf's or cell's mask run
@@ -50,30 +65,47 @@
 // every lane once any lane needs it. (Votes and warp barriers of the same kind
 // may be satisfied by lanes standing at different instructions, so a warp
 // whose lanes spent long, different times in divergent code was seen to fall
-// out of step.) Node and particle indices are checked before every gather; an
-// index out of range (which a valid tree never produces) sets kStatusInvalid
-// and is skipped.
+// out of step.) The conditions around the group's barriers are the same in
+// all its warps. Node slots and particle indices are checked before every
+// gather; an index out of range (which a valid tree never produces) sets
+// kStatusInvalid and is skipped.
+//
+// Bound by FP32 issue and the latency between dependent steps: at 200,000
+// particles (quadrupoles, two warps per group) the FMA pipe is 48 % busy and
+// 60 % of issue slots are used. Walk times, before (one warp per group, one
+// stack item per node) and after: 10,000 Plummer particles without quadrupoles
+// 360 -> 117 us; 100,000 collision particles 756 -> 666 us; 200,000 1.40 -> 1.32 ms;
+// 2,000,000 14.79 -> 14.42 ms. Relative error against 64 bits (2-norm): 10,000
+// 7.7e-8 -> 5.2e-8, 200,000 4.2e-8 -> 4.3e-8, 2,000,000 3.9e-8 -> 4.1e-8 (the
+// families of a batch pull the same way, so its FP32 partial sums are larger). Groups of 64 targets (two per lane) halve the
+// traversal but measured no faster at any size (2M 14.60 ms).
+#include <algorithm>
+#include <atomic>
+
 #include "common.cuh"
+#include "runtime.hpp"
 #include "tree_kernels.hpp"
 
 namespace ob {
 namespace {
 
-constexpr int kWalkWarps = 4;
-constexpr int kWalkThreads = kWalkWarps * 32;
 constexpr float kAcceptMargin = 4e-6f;
 constexpr uint32_t kFull = 0xffffffffu;
 
-// Per-warp shared-memory capacities (entries). A round takes at most 32 items;
-// each adds at most two stack items (its next sibling and, opened, its first
-// child) and at most one cell or one leaf, so a round of t items adds at most
-// 2t stack items, t cells and t leaves. A round takes at most stack room
-// (capacity - size) items, so the stack cannot overflow while it has room;
-// cells and leaves are evaluated once more than capacity - 32 are queued.
-// Sized so that 8 CTAs of 4 warps fit in an SM's shared memory.
+// Shared-memory capacities (entries). A stack item is a family: the children of
+// one opened node. A warp takes up to four families a round, one child per
+// lane; each child adds at most one family, one cell and one leaf. A round
+// takes at most as many families as the stack has room to push back (eight for
+// each one taken), so the stack cannot overflow while it has room; cells and
+// leaves are evaluated once more than capacity - 32 are queued.
+constexpr uint32_t kFamilies = 4;
 constexpr uint32_t kStackCap = 256;
 constexpr uint32_t kCellCap = 48;
 constexpr uint32_t kLeafCap = 40;
+// Cells summed in one FP32 chain.
+constexpr uint32_t kCellBlock = 16;
+// Leaves summed in FP32 before their sums are folded into FP64.
+constexpr uint32_t kLeafFold = 8;
 // Staged cell fields, as quads of packed pairs: quad f of pair p holds
 // (a_j, a_j+1, b_j, b_j+1) for the two fields a, b of group f and the cells
 // j = 2p, 2p+1: (x, y) (z, mass) (2.5 Qxx, 2.5 Qxy) (2.5 Qxz, 2.5 Qyy)
@@ -85,19 +117,38 @@ constexpr int kLeafQuads = 2;
 // terms it produces underflow to exactly zero in FP32.
 constexpr float kFar = 1e18f;
 
+// W warps share the traversal of a group of 32 targets (one per lane of each).
+template <int W> struct Shape {
+    static constexpr uint32_t groups = W == 1 ? 4u : 1u; // per CTA
+    static constexpr uint32_t threads = 32u * W * groups;
+    static constexpr uint32_t stack = kStackCap * (W < 4 ? W : 4);
+};
+
 struct __align__(16) WarpSpace {
     float4 cells[kCellQuads][kCellCap / 2 + 1]; // +1: the neutral partner of an odd count
     uint32_t cell_mask[kCellCap + 2];
-    float4 leaf_pos[kLeafCap];  // leaf centre of mass - G (FP32), particle count bits
-    uint2 leaf_meta[kLeafCap];  // (first particle | may-hold-a-target bit, target mask)
-    uint2 stack[kStackCap];     // (node, reach mask)
+    // Leaf centre of mass, FP32 hi with the particle count's bits and lo with
+    // those of the first particle | may-hold-a-target bit; target mask.
+    float4 leaf_hi[kLeafCap];
+    float4 leaf_lo[kLeafCap];
+    uint32_t leaf_mask[kLeafCap];
     union {                     // used one at a time
         float4 leaf_quads[kLeafQuads][17];
         float4 union_staged[32]; // the union walk's leaf staging (after a fallback)
     };
-    // Box of the warp's targets as FP32 hi + lo parts: lo hi, lo lo, hi hi,
+};
+
+template <int W> struct __align__(16) GroupSpace {
+    // Box of the group's targets as FP32 hi + lo parts: lo hi, lo lo, hi hi,
     // hi lo; then the box centre G hi, G lo (x, y, z; w unused).
     float4 box[6];
+    union {
+        WarpSpace warp[W];
+        double sums[W][3][32]; // the warps' sums, after the traversal (W > 1)
+    };
+    uint2 stack[Shape<W>::stack];        // first child's slot, mask of the targets that reach it
+    uint8_t stack_kids[Shape<W>::stack]; // number of children
+    uint32_t pushed[W]; // families a warp pushes this round
 };
 
 __device__ __forceinline__ float2 f2(float a, float b) { return make_float2(a, b); }
@@ -161,7 +212,7 @@ __device__ __forceinline__ bool lane_accepts(const float4 A, const float4 B, flo
 // FP32 partials), counts to pairs / cells.
 template <bool QUAD>
 __device__ void union_walk(const DeviceNode *__restrict__ nodes,
-                           const WalkNode *__restrict__ walk, const uint32_t *__restrict__ first_of,
+                           const DeviceQuadrupole *__restrict__ quads,
                            const float4 *__restrict__ leaf_rel, const double *__restrict__ sorted,
                            uint32_t n, uint32_t node_count, float eps2, uint32_t i, bool active,
                            float pxh, float pyh, float pzh, float pxl, float pyl, float pzl,
@@ -175,11 +226,16 @@ __device__ void union_walk(const DeviceNode *__restrict__ nodes,
         if (cur >= node_count) {
             break;
         }
-        const float4 A = walk[cur].a;
-        const float4 B = walk[cur].b;
-        const float4 D = walk[cur].d;
-        const uint32_t count = __float_as_uint(D.w) & kWalkCountMask;
-        const uint32_t next = count > 0u ? cur + 1u : __float_as_uint(D.z);
+        // The node's compact record, formed from its FP64 moments.
+        const DeviceNode cell = nodes[cur];
+        float4 A, B;
+        split(cell.com_x, A.x, B.x);
+        split(cell.com_y, A.y, B.y);
+        split(cell.com_z, A.z, B.z);
+        A.w = __double2float_rn(cell.mass);
+        B.w = __double2float_rn(cell.r2);
+        const uint32_t count = cell.count;
+        const uint32_t next = cell.next;
         bool open_leaf = false;
         float dx = 0.0f, dy = 0.0f, dz = 0.0f;
         if (cursor == cur) {
@@ -192,10 +248,13 @@ __device__ void union_walk(const DeviceNode *__restrict__ nodes,
                 const float f = (A.w * inv) * inv2;
                 float gx = dx * f, gy = dy * f, gz = dz * f;
                 if (QUAD) {
-                    const float4 C = walk[cur].c;
-                    const float qx = fmaf(C.x, dx, fmaf(C.y, dy, C.z * dz));
-                    const float qy = fmaf(C.y, dx, fmaf(C.w, dy, D.x * dz));
-                    const float qz = fmaf(C.z, dx, fmaf(D.x, dy, D.y * dz));
+                    const DeviceQuadrupole q = quads[cur];
+                    const float xx = __double2float_rn(q.xx), xy = __double2float_rn(q.xy);
+                    const float xz = __double2float_rn(q.xz), yy = __double2float_rn(q.yy);
+                    const float yz = __double2float_rn(q.yz), zz = __double2float_rn(q.zz);
+                    const float qx = fmaf(xx, dx, fmaf(xy, dy, xz * dz));
+                    const float qy = fmaf(xy, dx, fmaf(yy, dy, yz * dz));
+                    const float qz = fmaf(xz, dx, fmaf(yz, dy, zz * dz));
                     const float quadratic = fmaf(dx, qx, fmaf(dy, qy, dz * qz));
                     const float inv5 = (inv2 * inv2) * inv;
                     const float s = (2.5f * quadratic) * (inv5 * inv2);
@@ -216,7 +275,7 @@ __device__ void union_walk(const DeviceNode *__restrict__ nodes,
             }
         }
         if (__any_sync(kFull, open_leaf)) {
-            const uint32_t first = first_of[cur];
+            const uint32_t first = cell.first;
             const bool own = open_leaf && i >= first && i < first + count;
             const bool masked = __any_sync(kFull, own);
             float sx = 0.0f, sy = 0.0f, sz = 0.0f;
@@ -281,14 +340,17 @@ __device__ __forceinline__ void stage_cell(WarpSpace &ws, uint32_t j, float3 c, 
     ws.cell_mask[j] = mask;
 }
 
-// Queues opened leaf k: centre relative to G, size, first particle (with a
-// bit when its range may hold one of the warp's targets) and target mask.
-__device__ __forceinline__ void queue_leaf(WarpSpace &ws, uint32_t k, float3 c, uint32_t size,
-                                           uint32_t first, uint32_t mask, uint32_t warp_first,
-                                           uint32_t warp_end) {
-    const bool holds = first < warp_end && first + size > warp_first;
-    ws.leaf_pos[k] = make_float4(c.x, c.y, c.z, __uint_as_float(size));
-    ws.leaf_meta[k] = make_uint2(first | (holds ? 0x80000000u : 0u), mask);
+// Queues opened leaf k: centre of mass (hi + lo), size, first particle (with a
+// bit when its range may hold one of the group's targets) and target mask.
+__device__ __forceinline__ void queue_leaf(WarpSpace &ws, uint32_t k, const float4 A,
+                                           const float4 B, uint32_t size, uint32_t first,
+                                           uint32_t mask, uint32_t group_first,
+                                           uint32_t group_end) {
+    const bool holds = first < group_end && first + size > group_first;
+    ws.leaf_hi[k] = make_float4(A.x, A.y, A.z, __uint_as_float(size));
+    ws.leaf_lo[k] =
+        make_float4(B.x, B.y, B.z, __uint_as_float(first | (holds ? 0x80000000u : 0u)));
+    ws.leaf_mask[k] = mask;
 }
 
 // A leaf's first particle and size, checked against the particle count.
@@ -365,9 +427,18 @@ __device__ __forceinline__ void flush_cells(WarpSpace &ws, uint32_t count, float
         ws.cell_mask[count] = 0u;
     }
     __syncwarp();
+    // Blocks of cells are summed by themselves and then added to the batch's
+    // sums: shorter FP32 chains, smaller rounding.
     float2 sx = f2(0.0f, 0.0f), sy = sx, sz = sx;
-    for (uint32_t j = 0; j < count; j += 2) {
-        cell_pair<QUAD>(ws, j >> 1, ntx, nty, ntz, eps2, lane_bit, sx, sy, sz);
+    for (uint32_t from = 0; from < count; from += kCellBlock) {
+        const uint32_t to = min(from + kCellBlock, count);
+        float2 bx = f2(0.0f, 0.0f), by = bx, bz = bx;
+        for (uint32_t j = from; j < to; j += 2) {
+            cell_pair<QUAD>(ws, j >> 1, ntx, nty, ntz, eps2, lane_bit, bx, by, bz);
+        }
+        sx = __fadd2_rn(sx, bx);
+        sy = __fadd2_rn(sy, by);
+        sz = __fadd2_rn(sz, bz);
     }
     __syncwarp();
     acc_x += static_cast<double>(sx.x) + static_cast<double>(sx.y);
@@ -380,38 +451,47 @@ __device__ __forceinline__ void flush_cells(WarpSpace &ws, uint32_t count, float
 // leaf's mask sit far away and add exactly zero), two sources per FP32x2
 // instruction, skipping the target itself where the leaf's range may hold it.
 __device__ __forceinline__ void flush_leaves(WarpSpace &ws, uint32_t count,
-                                             const float4 *__restrict__ leaf_rel, float tgx,
-                                             float tgy, float tgz, float eps2, uint32_t i,
-                                             uint32_t lane_bit, double &acc_x, double &acc_y,
-                                             double &acc_z, uint32_t &pairs) {
+                                             const float4 *__restrict__ leaf_rel, float pxh,
+                                             float pyh, float pzh, float pxl, float pyl, float pzl,
+                                             float eps2, uint32_t i, uint32_t lane_bit,
+                                             double &acc_x, double &acc_y, double &acc_z,
+                                             uint32_t &pairs) {
     const uint32_t lane = threadIdx.x & 31u;
     const float2 e2 = f2(eps2, eps2);
     float2 sx = f2(0.0f, 0.0f), sy = sx, sz = sx;
     for (uint32_t k = 0; k < count; ++k) {
-        const float4 pos = ws.leaf_pos[k];
-        const uint2 e = ws.leaf_meta[k];
-        const uint32_t size = __float_as_uint(pos.w);
-        const uint32_t first = e.x & 0x7fffffffu;
-        const bool masked = (e.x >> 31) != 0u; // uniform: every lane reads the same entry
-        const bool in = (e.y & lane_bit) != 0u;
+        // Folded into FP64 every few leaves: shorter FP32 chains, smaller rounding.
+        if (k != 0u && (k & (kLeafFold - 1u)) == 0u) {
+            acc_x += static_cast<double>(sx.x) + static_cast<double>(sx.y);
+            acc_y += static_cast<double>(sy.x) + static_cast<double>(sy.y);
+            acc_z += static_cast<double>(sz.x) + static_cast<double>(sz.y);
+            sx = sy = sz = f2(0.0f, 0.0f);
+        }
+        const float4 hi = ws.leaf_hi[k], lo = ws.leaf_lo[k];
+        const uint32_t size = __float_as_uint(hi.w);
+        const uint32_t first = __float_as_uint(lo.w) & 0x7fffffffu;
+        // Uniform: every lane reads the same entry.
+        const bool masked = (__float_as_uint(lo.w) >> 31) != 0u;
+        const bool in = (ws.leaf_mask[k] & lane_bit) != 0u;
         const bool own = in && i >= first && i < first + size;
-        // Offset leaf centre of mass - target; source - target = source + d.
+        // Offset leaf centre of mass - target, from hi + lo parts (a few ulps of
+        // itself, however large the group's box); source - target = source + d.
         // Lanes outside the mask sit far away: their terms are exactly zero.
-        const float dx = in ? pos.x - tgx : kFar;
-        const float dy = in ? pos.y - tgy : kFar;
-        const float dz = in ? pos.z - tgz : kFar;
+        const float dx = in ? (hi.x - pxh) + (lo.x - pxl) : kFar;
+        const float dy = in ? (hi.y - pyh) + (lo.y - pyl) : kFar;
+        const float dz = in ? (hi.z - pzh) + (lo.z - pzl) : kFar;
         const float2 dx2 = f2(dx, dx), dy2 = f2(dy, dy), dz2 = f2(dz, dz);
         for (uint32_t base = 0; base < size; base += 32) {
             const uint32_t chunk = min(32u, size - base);
             float4(*lq)[17] = ws.leaf_quads;
+            float4 src = make_float4(kFar, kFar, kFar, 0.0f);
             if (lane < chunk) {
-                const float4 src = leaf_rel[first + base + lane];
+                src = leaf_rel[first + base + lane];
+            }
+            if (lane <= chunk) {
+                // Lane `chunk` adds the neutral partner: far away and massless.
                 put(lq[0], lane, src.x, src.y);
                 put(lq[1], lane, src.z, src.w);
-            } else if (lane == chunk) {
-                // Neutral partner: far away and massless.
-                put(lq[0], lane, kFar, kFar);
-                put(lq[1], lane, kFar, 0.0f);
             }
             __syncwarp();
             // Every lane runs the loop (no divergent region).
@@ -461,41 +541,57 @@ __device__ __forceinline__ void flush_leaves(WarpSpace &ws, uint32_t count,
     acc_z += static_cast<double>(sz.x) + static_cast<double>(sz.y);
 }
 
-template <bool QUAD>
-__global__ void __launch_bounds__(kWalkThreads, 8)
-    walk_kernel(const DeviceNode *__restrict__ nodes, const WalkNode *__restrict__ walk,
-                const uint32_t *__restrict__ first_of, const float4 *__restrict__ leaf_rel,
-                const double *__restrict__ sorted, const uint32_t *__restrict__ perm, uint32_t n,
-                float eps2, double *ax, double *ay, double *az, const TreeMeta *meta,
-                unsigned long long *counters, unsigned *status, uint32_t stack_cap) {
+// 28 warps per SM at 72 registers: with 32 at 64 the quadrupole walk spills
+// (2M 15.1 ms against 14.4), 24 at 80 hide less latency (15.0 ms).
+template <bool QUAD, int W>
+__global__ void __launch_bounds__(Shape<W>::threads, 896 / Shape<W>::threads)
+    walk_kernel(const DeviceNode *__restrict__ nodes,
+                const DeviceQuadrupole *__restrict__ quads, const float4 *__restrict__ walk_a,
+                const float4 *__restrict__ walk_b, const float4 *__restrict__ walk_c,
+                const float4 *__restrict__ walk_d, const uint32_t *__restrict__ walk_node,
+                const float4 *__restrict__ leaf_rel, const double *__restrict__ sorted,
+                const uint32_t *__restrict__ perm, uint32_t n, float eps2, double *ax, double *ay,
+                double *az, const TreeMeta *meta, unsigned long long *counters, unsigned *status,
+                uint32_t stack_cap) {
     extern __shared__ __align__(16) unsigned char smem[];
+    using Group = GroupSpace<W>;
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t warp = threadIdx.x >> 5;
-    WarpSpace &ws = reinterpret_cast<WarpSpace *>(smem)[warp];
-    const uint32_t i = (blockIdx.x * kWalkWarps + warp) * 32u + lane;
-    const bool active = i < n;
-    const uint32_t live = __ballot_sync(kFull, active);
-    if (live == 0u) {
-        return; // the whole warp lies past the last target
+    const uint32_t w = W == 1 ? 0u : warp; // this warp's place in its group
+    Group &gs = reinterpret_cast<Group *>(smem)[W == 1 ? warp : 0u];
+    WarpSpace &ws = gs.warp[w];
+    const uint32_t group = W == 1 ? blockIdx.x * Shape<W>::groups + warp : blockIdx.x;
+    // Past the last target: whole warps (W = 1) or no CTA at all (W > 1).
+    if (group >= ceil_div(n, 32u)) {
+        return;
     }
+    const uint32_t group_first = group * 32u;
+    const uint32_t group_end = min(group_first + 32u, n);
     const uint32_t node_count = meta->node_count;
     const uint32_t lane_bit = 1u << lane;
-    const uint32_t warp_first = i - lane;
-    const uint32_t warp_end = min(warp_first + 32u, n);
+    const float2 eps2v = f2(eps2, eps2);
+    auto group_sync = [] {
+        if constexpr (W == 1) {
+            __syncwarp();
+        } else {
+            __syncthreads();
+        }
+    };
 
+    // The lane's target, and the FP64 bounding box of the group's.
+    const uint32_t i = group_first + lane;
+    const bool active = i < n;
+    const uint32_t live = __ballot_sync(kFull, active);
     double X = 0.0, Y = 0.0, Z = 0.0;
-    float pxh = 0.0f, pyh = 0.0f, pzh = 0.0f, pxl = 0.0f, pyl = 0.0f, pzl = 0.0f;
     if (active) {
         X = sorted[i];
         Y = sorted[static_cast<size_t>(n) + i];
         Z = sorted[2ull * n + i];
-        split(X, pxh, pxl);
-        split(Y, pyh, pyl);
-        split(Z, pzh, pzl);
     }
-    const float2 eps2v = f2(eps2, eps2);
-
-    // FP64 bounding box of the warp's targets.
+    float pxh, pyh, pzh, pxl, pyl, pzl;
+    split(X, pxh, pxl);
+    split(Y, pyh, pyl);
+    split(Z, pzh, pzl);
     const double inf = __longlong_as_double(0x7ff0000000000000ll);
     double lox = active ? X : inf, loy = active ? Y : inf, loz = active ? Z : inf;
     double hix = active ? X : -inf, hiy = active ? Y : -inf, hiz = active ? Z : -inf;
@@ -513,7 +609,7 @@ __global__ void __launch_bounds__(kWalkThreads, 8)
     const float tgx = __double2float_rn(X - gcx), tgy = __double2float_rn(Y - gcy),
                 tgz = __double2float_rn(Z - gcz);
     const float2 ntx = f2(-tgx, -tgx), nty = f2(-tgy, -tgy), ntz = f2(-tgz, -tgz);
-    if (lane < 6) {
+    if (w == 0 && lane < 6) {
         // Lanes 0-5 split one box value each: lo, hi, G (x, y, z).
         const double v[3] = {lane < 2 ? lox : lane < 4 ? hix : gcx,
                              lane < 2 ? loy : lane < 4 ? hiy : gcy,
@@ -523,38 +619,45 @@ __global__ void __launch_bounds__(kWalkThreads, 8)
             split(v[a], h[a], l[a]);
         }
         // Slots: 0 lo hi, 1 lo lo, 2 hi hi, 3 hi lo, 4 G hi, 5 G lo.
-        ws.box[lane] = (lane & 1u) == 0u ? make_float4(h[0], h[1], h[2], 0.0f)
-                                          : make_float4(l[0], l[1], l[2], 0.0f);
+        gs.box[lane] = (lane & 1u) == 0u ? make_float4(h[0], h[1], h[2], 0.0f)
+                                         : make_float4(l[0], l[1], l[2], 0.0f);
     }
-    __syncwarp();
 
     double acc_x = 0.0, acc_y = 0.0, acc_z = 0.0;
     uint32_t pairs = 0, cells = 0;
     uint32_t size = 1, ncell = 0, nleaf = 0;
     bool overflow = false;
     uint32_t rounds = 0;
-    if (lane == 0) {
-        ws.stack[0] = make_uint2(0u, live);
+    if (w == 0 && lane == 0) {
+        gs.stack[0] = make_uint2(0u, live); // the root, a family of one
+        gs.stack_kids[0] = 1u;
     }
-    __syncwarp();
+    group_sync();
     while (size > 0) {
-        // Popping t items and pushing up to 2t needs size + t <= stack_cap.
-        const uint32_t take = min(min(size, 32u), stack_cap - min(size, stack_cap));
+        // Popping t families and pushing up to 8t needs size + 7t <= stack_cap.
+        const uint32_t take = min(min(size, kFamilies * W), (stack_cap - min(size, stack_cap)) / 7u);
         // A valid tree visits each node at most once, so more rounds than
-        // nodes (or a full stack) hands the warp to the union walk, whose
+        // nodes (or a full stack) hands the group to the union walk, whose
         // cursors only move forward.
         if (take == 0u || ++rounds > node_count + 1u) {
-            overflow = true;
+            overflow = true; // the same in every warp of the group
             break;
         }
         size -= take;
-        const bool has = lane < take;
-        uint2 item = make_uint2(0u, 0u);
-        if (has) {
-            item = ws.stack[size + lane];
-            if (item.x >= node_count) {
+        // Family w, w + W, ... of the round for warp w; lane 8f + k takes
+        // child k of the warp's f-th.
+        const uint32_t family = (lane >> 3) * W + w;
+        bool has = false;
+        uint32_t slot = 0u, reach = 0u;
+        if (family < take) {
+            const uint32_t at = size + family;
+            has = (lane & 7u) < gs.stack_kids[at];
+            const uint2 item = gs.stack[at];
+            slot = item.x + (lane & 7u);
+            reach = item.y;
+            if (has && slot >= node_count) {
                 atomicOr(status, kStatusInvalid);
-                item.x = node_count; // skipped below
+                has = false;
             }
         }
         __syncwarp();
@@ -562,18 +665,16 @@ __global__ void __launch_bounds__(kWalkThreads, 8)
         // Classify the lane's node against the box from its compact record:
         // every target accepts it (cell_mask = the item's mask), every target
         // opens it (open_mask), or each target decides for itself (mixed).
-        bool sibling = false, mixed = false;
-        uint32_t next = 0, count = 0, cell_mask = 0u, open_mask = 0u;
+        bool mixed = false;
+        uint32_t word = 0u; // a leaf's bit and count, or the number of children
+        uint32_t cell_mask = 0u, open_mask = 0u;
         float4 A = make_float4(0.0f, 0.0f, 0.0f, 0.0f), B = A, C = A, D = A;
-        if (has && item.x < node_count) {
-            A = walk[item.x].a;
-            B = walk[item.x].b;
-            D = walk[item.x].d;
-            const uint32_t word = __float_as_uint(D.w);
-            count = word & kWalkCountMask;
-            next = count > 0u ? item.x + 1u : __float_as_uint(D.z);
-            sibling = (word & kWalkSiblingBit) != 0u;
-            const float4 loh = ws.box[0], lol = ws.box[1], hih = ws.box[2], hil = ws.box[3];
+        if (has) {
+            A = walk_a[slot];
+            B = walk_b[slot];
+            D = walk_d[slot];
+            word = __float_as_uint(D.w);
+            const float4 loh = gs.box[0], lol = gs.box[1], hih = gs.box[2], hil = gs.box[3];
             // Signed distances lo - c and c - hi per axis, from hi + lo parts.
             const float lx = (loh.x - A.x) + (lol.x - B.x), ux = (A.x - hih.x) + (B.x - hil.x);
             const float ly = (loh.y - A.y) + (lol.y - B.y), uy = (A.y - hih.y) + (B.y - hil.y);
@@ -588,31 +689,26 @@ __global__ void __launch_bounds__(kWalkThreads, 8)
             const float far2 = fmaf(fz, fz, fmaf(fy, fy, fx * fx));
             const float r2 = B.w;
             if (near2 >= r2 * (1.0f + kAcceptMargin) && r2 > 1e-30f) {
-                cell_mask = item.y;
+                cell_mask = reach;
             } else if (far2 < r2 * (1.0f - kAcceptMargin)) {
-                open_mask = item.y;
+                open_mask = reach;
             } else {
                 mixed = true;
             }
         }
         const uint32_t below = lanes_below(lane);
-        const uint32_t bs = __ballot_sync(kFull, sibling);
-        if (sibling) {
-            ws.stack[size + __popc(bs & below)] = make_uint2(next, item.y);
-        }
-        size += __popc(bs);
 
         // Mixed nodes: each target in the mask decides for itself; the lane
         // that classified the node keeps the accepted and opened masks.
         for (uint32_t bm = __ballot_sync(kFull, mixed); bm != 0u; bm &= bm - 1u) {
             const uint32_t owner = __ffs(bm) - 1u;
-            const uint32_t v = __shfl_sync(kFull, item.x, owner);
-            const uint32_t mask = __shfl_sync(kFull, item.y, owner);
-            const float4 MA = walk[v].a;
-            const float4 MB = walk[v].b;
+            const uint32_t v = __shfl_sync(kFull, slot, owner);
+            const float4 MA = walk_a[v];
+            const float4 MB = walk_b[v];
+            const uint32_t mask = __shfl_sync(kFull, reach, owner);
             // FP32 test on every lane; the FP64 test, when any lane of the
             // mask falls inside the margin, on every lane too.
-            const bool reach = (mask & lane_bit) != 0u;
+            const bool reached = (mask & lane_bit) != 0u;
             const float dx = (MA.x - pxh) + (MB.x - pxl);
             const float dy = (MA.y - pyh) + (MB.y - pyl);
             const float dz = (MA.z - pzh) + (MB.z - pzl);
@@ -620,10 +716,10 @@ __global__ void __launch_bounds__(kWalkThreads, 8)
             const float r2 = MB.w;
             const bool sure_accept = d2 >= r2 * (1.0f + kAcceptMargin) && r2 > 1e-30f;
             const bool sure_open = d2 <= r2 * (1.0f - kAcceptMargin);
-            bool accept = reach && sure_accept;
-            const bool unsure = reach && !sure_accept && !sure_open;
+            bool accept = reached && sure_accept;
+            const bool unsure = reached && !sure_accept && !sure_open;
             if (__any_sync(kFull, unsure)) {
-                const bool exact = exact_accept(nodes, v, sorted, n, active ? i : 0u);
+                const bool exact = exact_accept(nodes, walk_node[v], sorted, n, active ? i : 0u);
                 accept = accept || (unsure && exact);
             }
             const uint32_t accepted = __ballot_sync(kFull, accept) & mask;
@@ -634,68 +730,104 @@ __global__ void __launch_bounds__(kWalkThreads, 8)
         }
 
         // Every lane files its node's outcome: a staged cell for the targets
-        // that accept it, and for those that open it a queued leaf or a pushed
-        // first child.
+        // that accept it, and for those that open it a queued leaf or the
+        // pushed family of its children.
         const bool cell = cell_mask != 0u;
-        const bool leaf = open_mask != 0u && count > 0u;
-        const bool child = open_mask != 0u && count == 0u;
+        const bool opened = open_mask != 0u;
+        const bool leaf = opened && (word & kWalkLeafBit) != 0u;
+        const bool push = opened && (word & kWalkLeafBit) == 0u;
         const uint32_t ba = __ballot_sync(kFull, cell);
         const uint32_t bl = __ballot_sync(kFull, leaf);
-        const uint32_t bc = __ballot_sync(kFull, child);
-        if (child) {
-            ws.stack[size + __popc(bc & below)] = make_uint2(item.x + 1u, open_mask);
-        }
-        if (cell || leaf) {
-            const float4 Gh = ws.box[4], Gl = ws.box[5];
-            const float3 c = centre_rel(A, B, Gh, Gl);
-            if (cell) {
-                if (QUAD) {
-                    C = walk[item.x].c;
-                }
-                stage_cell<QUAD>(ws, ncell + __popc(ba & below), c, A.w, cell_mask, C, D);
-                cells += __popc(cell_mask); // every target of the mask takes the cell
+        const uint32_t bc = __ballot_sync(kFull, push);
+        uint32_t at = size, total = __popc(bc);
+        if constexpr (W > 1) {
+            if (lane == 0) {
+                gs.pushed[w] = total;
             }
-            if (leaf) {
-                uint32_t first, lsize;
-                leaf_range(__float_as_uint(D.z), count, n, status, first, lsize);
-                queue_leaf(ws, nleaf + __popc(bl & below), c, lsize, first, open_mask,
-                           warp_first, warp_end);
+            __syncthreads(); // the counts are written and every item of the round is read
+            total = 0u;
+#pragma unroll
+            for (uint32_t q = 0; q < W; ++q) {
+                const uint32_t c = gs.pushed[q];
+                at += q < w ? c : 0u;
+                total += c;
             }
         }
-        size += __popc(bc);
+        if (push) {
+            at += __popc(bc & below);
+            gs.stack[at] = make_uint2(__float_as_uint(D.z), open_mask);
+            gs.stack_kids[at] = static_cast<uint8_t>(min(word, 8u));
+        }
+        if (cell) {
+            if (QUAD) {
+                C = walk_c[slot];
+            }
+            stage_cell<QUAD>(ws, ncell + __popc(ba & below),
+                             centre_rel(A, B, gs.box[4], gs.box[5]), A.w, cell_mask, C, D);
+            cells += __popc(cell_mask); // every target of the mask takes the cell
+        }
+        if (leaf) {
+            uint32_t first, lsize;
+            leaf_range(__float_as_uint(D.z), word & ~kWalkLeafBit, n, status, first, lsize);
+            queue_leaf(ws, nleaf + __popc(bl & below), A, B, lsize, first, open_mask,
+                       group_first, group_end);
+        }
+        size += total;
         ncell += __popc(ba);
         nleaf += __popc(bl);
-        __syncwarp();
+        group_sync();
         if (ncell > kCellCap - 32u) {
             flush_cells<QUAD>(ws, ncell, ntx, nty, ntz, eps2v, lane_bit, acc_x, acc_y, acc_z);
             ncell = 0;
         }
         if (nleaf > kLeafCap - 32u) {
-            flush_leaves(ws, nleaf, leaf_rel, tgx, tgy, tgz, eps2, i, lane_bit, acc_x, acc_y,
-                         acc_z, pairs);
+            flush_leaves(ws, nleaf, leaf_rel, pxh, pyh, pzh, pxl, pyl, pzl, eps2, i, lane_bit,
+                         acc_x, acc_y, acc_z, pairs);
             nleaf = 0;
         }
     }
     if (overflow) {
         acc_x = acc_y = acc_z = 0.0;
         pairs = cells = 0;
-        union_walk<QUAD>(nodes, walk, first_of, leaf_rel, sorted, n, node_count, eps2, i, active,
-                         pxh, pyh, pzh, pxl, pyl, pzl, ws.union_staged, acc_x, acc_y, acc_z, pairs,
-                         cells);
+        if (w == 0) { // the group's other warps add nothing
+            union_walk<QUAD>(nodes, quads, leaf_rel, sorted, n, node_count, eps2, i, active, pxh,
+                             pyh, pzh, pxl, pyl, pzl, ws.union_staged, acc_x, acc_y, acc_z, pairs,
+                             cells);
+        }
     } else {
         flush_cells<QUAD>(ws, ncell, ntx, nty, ntz, eps2v, lane_bit, acc_x, acc_y, acc_z);
-        flush_leaves(ws, nleaf, leaf_rel, tgx, tgy, tgz, eps2, i, lane_bit, acc_x, acc_y, acc_z,
-                     pairs);
+        flush_leaves(ws, nleaf, leaf_rel, pxh, pyh, pzh, pxl, pyl, pzl, eps2, i, lane_bit,
+                         acc_x, acc_y, acc_z, pairs);
     }
 
-    if (active) {
-        const uint32_t j = perm[i];
-        ax[j] = acc_x;
-        ay[j] = acc_y;
-        az[j] = acc_z;
+    if constexpr (W == 1) {
+        if (active) {
+            const uint32_t j = perm[i];
+            ax[j] = acc_x;
+            ay[j] = acc_y;
+            az[j] = acc_z;
+        }
+    } else {
+        // The warps' sums, added in warp order: component w by warp w (and by
+        // warps 0 and 1 in turn when the group has two).
+        __syncthreads();
+        gs.sums[w][0][lane] = acc_x;
+        gs.sums[w][1][lane] = acc_y;
+        gs.sums[w][2][lane] = acc_z;
+        __syncthreads();
+        for (uint32_t k = w; k < 3u; k += W) {
+            double sum = gs.sums[0][k][lane];
+#pragma unroll
+            for (uint32_t q = 1; q < W; ++q) {
+                sum += gs.sums[q][k][lane];
+            }
+            if (active) {
+                (k == 0u ? ax : k == 1u ? ay : az)[perm[i]] = sum;
+            }
+        }
     }
     // pairs: per target; cells: tallied by the lanes that queued the entries.
-    unsigned long long p = active ? pairs : 0u, c = cells;
+    unsigned long long p = pairs, c = cells;
     for (int off = 16; off > 0; off >>= 1) {
         p += __shfl_down_sync(kFull, p, off);
         c += __shfl_down_sync(kFull, c, off);
@@ -710,29 +842,78 @@ __global__ void __launch_bounds__(kWalkThreads, 8)
 
 uint32_t walk_stack_capacity() { return kStackCap; }
 
-cudaError_t launch_walk(const DeviceNode *nodes, const WalkNode *walk_nodes,
-                        const uint32_t *first_of, const float4 *leaf_rel, const double *sorted,
-                        const uint32_t *perm, uint32_t n, double eps2, bool quadrupole,
-                        double *ax, double *ay, double *az, TreeMeta *meta,
-                        unsigned long long *counters, unsigned *status, cudaStream_t stream,
-                        uint32_t stack_cap) {
+namespace {
+
+struct WalkArgs {
+    const DeviceNode *nodes;
+    const DeviceQuadrupole *quads;
+    WalkNodes walk;
+    const float4 *leaf_rel;
+    const double *sorted;
+    const uint32_t *perm;
+    uint32_t n;
+    float eps2;
+    double *ax, *ay, *az;
+    TreeMeta *meta;
+    unsigned long long *counters;
+    unsigned *status;
+    uint32_t stack_cap;
+};
+
+template <bool QUAD, int W> cudaError_t launch_shape(const WalkArgs &a, cudaStream_t stream) {
+    using S = Shape<W>;
+    const uint32_t cap = a.stack_cap == 0u ? S::stack : std::min(a.stack_cap, S::stack);
+    const uint32_t blocks = ceil_div(ceil_div(a.n, 32u), S::groups);
+    const size_t smem = S::groups * sizeof(GroupSpace<W>);
+    static std::atomic<uint64_t> configured{0};
+    auto kernel = walk_kernel<QUAD, W>;
+    const cudaError_t err = set_smem_limit_once(reinterpret_cast<const void *>(kernel),
+                                                static_cast<int>(smem), configured);
+    if (err != cudaSuccess) {
+        return err;
+    }
+    kernel<<<blocks, S::threads, smem, stream>>>(
+        a.nodes, a.quads, a.walk.a, a.walk.b, a.walk.c, a.walk.d, a.walk.node, a.leaf_rel,
+        a.sorted, a.perm, a.n, a.eps2, a.ax, a.ay, a.az, a.meta, a.counters, a.status, cap);
+    return cudaGetLastError();
+}
+
+// Warps per group: the most (up to 8) that keep the launch within about 3.5
+// times the warps resident on 148 SMs. Measured walks of the collision
+// (quadrupoles) with 1, 2, 4 and 8 warps per group: 30,000 particles 428, 301,
+// 204, 197 us; 100,000 758, 682, 645, 684 us; 200,000 1.38, 1.31, 1.33, 1.55 ms;
+// 500,000 3.48, 3.52, 3.74, 4.35 ms (sixteen warps: 98 us against 96 at 10,000,
+// and slower above).
+constexpr uint64_t kWarpsWanted = 16384;
+
+template <bool QUAD> cudaError_t launch_quad(const WalkArgs &a, cudaStream_t stream) {
+    const uint64_t groups = ceil_div(a.n, 32u);
+    if (8u * groups <= kWarpsWanted) {
+        return launch_shape<QUAD, 8>(a, stream);
+    }
+    if (4u * groups <= kWarpsWanted) {
+        return launch_shape<QUAD, 4>(a, stream);
+    }
+    if (2u * groups <= kWarpsWanted) {
+        return launch_shape<QUAD, 2>(a, stream);
+    }
+    return launch_shape<QUAD, 1>(a, stream);
+}
+
+} // namespace
+
+cudaError_t launch_walk(const DeviceNode *nodes, const DeviceQuadrupole *quads,
+                        const WalkNodes &walk, const float4 *leaf_rel, const double *sorted,
+                        const uint32_t *perm, uint32_t n, double eps2, double *ax, double *ay,
+                        double *az, TreeMeta *meta, unsigned long long *counters,
+                        unsigned *status, cudaStream_t stream, uint32_t stack_cap) {
     if (n == 0) {
         return cudaSuccess;
     }
-    const uint32_t cap = stack_cap == 0u || stack_cap > kStackCap ? kStackCap : stack_cap;
-    const uint32_t blocks = ceil_div(n, static_cast<uint32_t>(kWalkThreads));
-    const float eps2f = static_cast<float>(eps2);
-    const size_t smem = kWalkWarps * sizeof(WarpSpace);
-    if (quadrupole) {
-        walk_kernel<true><<<blocks, kWalkThreads, smem, stream>>>(
-            nodes, walk_nodes, first_of, leaf_rel, sorted, perm, n, eps2f, ax, ay, az, meta,
-            counters, status, cap);
-    } else {
-        walk_kernel<false><<<blocks, kWalkThreads, smem, stream>>>(
-            nodes, walk_nodes, first_of, leaf_rel, sorted, perm, n, eps2f, ax, ay, az, meta,
-            counters, status, cap);
-    }
-    return cudaGetLastError();
+    const auto eps2f = static_cast<float>(eps2);
+    const WalkArgs args{nodes, quads, walk, leaf_rel, sorted,   perm,   n, eps2f,
+                        ax,    ay,    az,   meta,     counters, status, stack_cap};
+    return quads != nullptr ? launch_quad<true>(args, stream) : launch_quad<false>(args, stream);
 }
 
 } // namespace ob

@@ -92,6 +92,27 @@ def test_ragged_sizes_and_parameters_against_oracle(b200, restatement, n, leaf, 
         assert a.tolist() == [[0.0, 0.0, 0.0]]
 
 
+# 65,536, 131,072 and 262,144 targets are the most that 8, 4 and 2 warps per
+# group of 32 take; a second group starts at 33.
+@pytest.mark.parametrize("n,quad", [(31, True), (32, False), (33, True), (65536, True),
+                                    (65537, False), (131073, True), (262144, False),
+                                    (262145, True)])
+def test_every_number_of_warps_per_group_gives_the_oracle_s_counts(b200, restatement, n, quad):
+    from orrery_b200 import initial_conditions as ic
+    d = ic.plummer_sphere(n, seed=n)
+    x, y, z, m = _xyzm(d)
+    s = b200.B200TreeSolver(0.02, 1.0, 24, quad)
+    a = s.evaluate((x, y, z), m)
+    a_ref, counts = restatement.barnes_hut(x, y, z, m, 0.02, 1.0, 24, quad)
+    c = s.interaction_count()
+    assert (c.particle_particle, c.particle_cell) == (counts.particle_particle,
+                                                      counts.particle_cell)
+    err = relative_errors(a, a_ref)
+    assert err.max() < TREE_WORST and np.sqrt((err ** 2).mean()) < 1e-5
+    again = s.evaluate((x, y, z), m)
+    assert np.array_equal(a, again)  # the warps' sums are added in a fixed order
+
+
 # --------------------------------------------------------------------------
 # The FP64 parity mode: forces equal to BarnesHutSolver's bit for bit
 # --------------------------------------------------------------------------
