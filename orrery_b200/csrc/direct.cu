@@ -26,6 +26,8 @@
 #include <type_traits>
 
 #include "common.cuh"
+#include "f64_math.cuh"
+#include "f64_ordered.cuh"
 #include "runtime.hpp"
 #include "internal.hpp"
 #include "split_math.cuh"
@@ -473,60 +475,172 @@ __global__ void __launch_bounds__(THREADS) direct_split_kernel(const DirectArgs 
 // (src/solvers/direct_kernel_scalar.cpp:31-59) with the split at i of
 // DirectSolver::evaluate (src/solvers/direct_solver.cpp:49-56): every operation
 // is an explicitly rounded FP64 intrinsic, so nothing is contracted and the
-// result is bit-identical to the reference's scalar kernel.
-constexpr int kF64Threads = 128;
-constexpr int kF64Tile = 256;
+// result is bit-identical to the reference's scalar kernel. The terms of a
+// target are formed by many warps and added in index order (f64_ordered.cuh).
+struct ForceTerm {
+    static constexpr int components = 3;
+    static constexpr int warps = 16; // 4,096 targets: 78 us, with 8 warps 89 us
+    static __device__ __forceinline__ void form(double m, double inv, double dx, double dy,
+                                                double dz, double (&term)[3]) {
+        const double f = __dmul_rn(m, __dmul_rn(__dmul_rn(inv, inv), inv));
+        term[0] = __dmul_rn(f, dx);
+        term[1] = __dmul_rn(f, dy);
+        term[2] = __dmul_rn(f, dz);
+    }
+};
 
-__global__ void __launch_bounds__(kF64Threads)
+__global__ void __launch_bounds__(OrderedShape<ForceTerm>::threads)
     direct_f64_kernel(const double *__restrict__ x, const double *__restrict__ y,
                       const double *__restrict__ z, const double *__restrict__ m, uint32_t n,
                       double eps2, double *ax, double *ay, double *az) {
-    __shared__ double tx[kF64Tile], ty[kF64Tile], tz[kF64Tile], tm[kF64Tile];
-    const uint32_t i = blockIdx.x * kF64Threads + threadIdx.x;
-    const bool valid = i < n;
-    const double px = valid ? x[i] : 0.0;
-    const double py = valid ? y[i] : 0.0;
-    const double pz = valid ? z[i] : 0.0;
-    double bx = 0.0, by = 0.0, bz = 0.0; // sources before i
-    double fx = 0.0, fy = 0.0, fz = 0.0; // sources after i
-    for (uint32_t base = 0; base < n; base += kF64Tile) {
-        for (uint32_t k = threadIdx.x; k < kF64Tile; k += kF64Threads) {
-            const uint32_t j = base + k;
-            tx[k] = j < n ? x[j] : 0.0;
-            ty[k] = j < n ? y[j] : 0.0;
-            tz[k] = j < n ? z[j] : 0.0;
-            tm[k] = j < n ? m[j] : 0.0;
-        }
-        __syncthreads();
-        const uint32_t count = min(static_cast<uint32_t>(kF64Tile), n - base);
-        for (uint32_t k = 0; k < count; ++k) {
-            const uint32_t j = base + k;
-            if (j == i) {
-                continue;
+    extern __shared__ __align__(16) unsigned char smem[];
+    auto &space = *reinterpret_cast<OrderedSpace<ForceTerm> *>(smem);
+    const uint32_t own = blockIdx.x; // the chunk that holds this CTA's targets
+    const uint32_t lane = threadIdx.x & 31u;
+    double before = 0.0, sum = 0.0; // sources before the target, then after it
+    ordered_terms<ForceTerm>(
+        space, x, y, z, m, n, eps2, own, 0u,
+        [&](uint32_t chunk, uint32_t count, const double2 *terms) {
+            if (chunk != own) {
+                add_chunk(sum, terms, count);
+                return;
             }
-            const double dx = __dsub_rn(tx[k], px);
-            const double dy = __dsub_rn(ty[k], py);
-            const double dz = __dsub_rn(tz[k], pz);
-            const double s2 =
-                __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz));
-            const double inv = __ddiv_rn(1.0, __dsqrt_rn(__dadd_rn(s2, eps2)));
-            const double f = __dmul_rn(tm[k], __dmul_rn(__dmul_rn(inv, inv), inv));
-            if (j < i) {
-                bx = __dadd_rn(bx, __dmul_rn(f, dx));
-                by = __dadd_rn(by, __dmul_rn(f, dy));
-                bz = __dadd_rn(bz, __dmul_rn(f, dz));
-            } else {
-                fx = __dadd_rn(fx, __dmul_rn(f, dx));
-                fy = __dadd_rn(fy, __dmul_rn(f, dy));
-                fz = __dadd_rn(fz, __dmul_rn(f, dz));
+            for (uint32_t k = 0; k < count; ++k) {
+                const double t = chunk_term(terms, k);
+                if (k == lane) {
+                    before = sum;
+                    sum = 0.0;
+                } else {
+                    sum = __dadd_rn(sum, t);
+                }
             }
-        }
-        __syncthreads();
+        });
+    const uint32_t component = threadIdx.x >> 5;
+    const uint32_t i = own * kOrderedTargets + lane;
+    if (component < 3u && i < n) {
+        (component == 0u ? ax : component == 1u ? ay : az)[i] = __dadd_rn(before, sum);
     }
-    if (valid) {
-        ax[i] = __dadd_rn(bx, fx);
-        ay[i] = __dadd_rn(by, fy);
-        az[i] = __dadd_rn(bz, fz);
+}
+
+// The same sums with one target per thread and no exchange between warps, for
+// systems large enough to give every SM sub-partition a warp: the terms of
+// kAhead sources are formed side by side, so that their dependent chains
+// overlap, and added in index order. Each warp stages its own sources.
+constexpr uint32_t kAhead = 4;
+constexpr uint32_t kWideThreads = 64;
+// From here on one target per thread: with the terms formed by many warps,
+// and one target per thread, an evaluation took 242 and 482 us at 8,192
+// targets, 898 and 952 us at 16,384 (0.9 warps per SM sub-partition), 3.08 and
+// 2.66 ms at 32,768 (shared memory carries 48 bytes per pair there), 12.1 and
+// 9.9 ms at 65,536. The former single kernel (one target per thread, the
+// general root and division, 128-thread CTAs): 731 us at 4,096, 2.91 ms at
+// 16,384, 15.3 ms at 65,536.
+constexpr uint32_t kWideFrom = 16384;
+
+__global__ void __launch_bounds__(kWideThreads)
+    direct_f64_wide_kernel(const double *__restrict__ x, const double *__restrict__ y,
+                           const double *__restrict__ z, const double *__restrict__ m, uint32_t n,
+                           double eps2, double *ax, double *ay, double *az) {
+    __shared__ double staged[kWideThreads / 32][2][4][32];
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t own = blockIdx.x * (kWideThreads / 32) + (threadIdx.x >> 5); // targets' chunk
+    const uint32_t i = own * 32u + lane;
+    if (own * 32u >= n) {
+        return; // the whole warp lies past the last target; warps do not wait on one another
+    }
+    double(*tile)[4][32] = staged[threadIdx.x >> 5];
+    const double px = i < n ? x[i] : 0.0, py = i < n ? y[i] : 0.0, pz = i < n ? z[i] : 0.0;
+    double bx = 0.0, by = 0.0, bz = 0.0; // sources before i
+    double sx = 0.0, sy = 0.0, sz = 0.0; // sources after the last reset
+    const uint32_t chunks = (n + 31u) / 32u;
+    double next[4] = {0.0, 0.0, 0.0, 0.0};
+    auto fetch = [&](uint32_t chunk) {
+        const uint32_t j = chunk * 32u + lane;
+        const bool real = chunk < chunks && j < n;
+        next[0] = real ? x[j] : 0.0;
+        next[1] = real ? y[j] : 0.0;
+        next[2] = real ? z[j] : 0.0;
+        next[3] = real ? m[j] : 0.0;
+    };
+    fetch(0u);
+    for (uint32_t c = 0; c < chunks; ++c) {
+        double(*src)[32] = tile[c & 1u];
+#pragma unroll
+        for (int a = 0; a < 4; ++a) {
+            src[a][lane] = next[a];
+        }
+        __syncwarp();
+        fetch(c + 1u);
+        const uint32_t count = min(32u, n - c * 32u);
+        const uint32_t groups = count / kAhead * kAhead;
+        auto one = [&](uint32_t k) {
+            const double dx = __dsub_rn(src[0][k], px);
+            const double dy = __dsub_rn(src[1][k], py);
+            const double dz = __dsub_rn(src[2][k], pz);
+            const double r2 = __dadd_rn(
+                __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz)),
+                eps2);
+            double t[3];
+            ForceTerm::form(src[3][k], inverse_root(r2), dx, dy, dz, t);
+            if (c == own && k == lane) { // the target itself: the sums start again
+                bx = sx;
+                by = sy;
+                bz = sz;
+                sx = sy = sz = 0.0;
+            } else {
+                sx = __dadd_rn(sx, t[0]);
+                sy = __dadd_rn(sy, t[1]);
+                sz = __dadd_rn(sz, t[2]);
+            }
+        };
+        if (c == own) {
+            for (uint32_t k = 0; k < count; ++k) {
+                one(k);
+            }
+            continue;
+        }
+        for (uint32_t k0 = 0; k0 < groups; k0 += kAhead) {
+            double dx[kAhead], dy[kAhead], dz[kAhead], r2[kAhead], inv[kAhead];
+            bool in_range = true;
+#pragma unroll
+            for (uint32_t k = 0; k < kAhead; ++k) {
+                dx[k] = __dsub_rn(src[0][k0 + k], px);
+                dy[k] = __dsub_rn(src[1][k0 + k], py);
+                dz[k] = __dsub_rn(src[2][k0 + k], pz);
+                r2[k] = __dadd_rn(__dadd_rn(__dadd_rn(__dmul_rn(dx[k], dx[k]),
+                                                      __dmul_rn(dy[k], dy[k])),
+                                            __dmul_rn(dz[k], dz[k])),
+                                  eps2);
+                in_range = in_range && inverse_root_in_range(r2[k]);
+            }
+            if (__all_sync(0xffffffffu, in_range)) {
+#pragma unroll
+                for (uint32_t k = 0; k < kAhead; ++k) {
+                    inv[k] = inverse_root_in_range_rn(r2[k]);
+                }
+            } else {
+#pragma unroll
+                for (uint32_t k = 0; k < kAhead; ++k) {
+                    inv[k] = inverse_root_general(r2[k]);
+                }
+            }
+#pragma unroll
+            for (uint32_t k = 0; k < kAhead; ++k) {
+                double t[3];
+                ForceTerm::form(src[3][k0 + k], inv[k], dx[k], dy[k], dz[k], t);
+                sx = __dadd_rn(sx, t[0]);
+                sy = __dadd_rn(sy, t[1]);
+                sz = __dadd_rn(sz, t[2]);
+            }
+        }
+        for (uint32_t k = groups; k < count; ++k) {
+            one(k);
+        }
+    }
+    if (i < n) {
+        ax[i] = __dadd_rn(bx, sx);
+        ay[i] = __dadd_rn(by, sy);
+        az[i] = __dadd_rn(bz, sz);
     }
 }
 
@@ -684,8 +798,21 @@ cudaError_t launch_direct_f64(const double *x, const double *y, const double *z,
     if (n == 0) {
         return cudaSuccess;
     }
-    direct_f64_kernel<<<ceil_div(n, kF64Threads), kF64Threads, 0, stream>>>(x, y, z, m, n, eps2,
-                                                                          ax, ay, az);
+    if (n >= kWideFrom) {
+        direct_f64_wide_kernel<<<ceil_div(n, kWideThreads), kWideThreads, 0, stream>>>(
+            x, y, z, m, n, eps2, ax, ay, az);
+        return cudaGetLastError();
+    }
+    static std::atomic<uint64_t> configured{0};
+    constexpr size_t smem = sizeof(OrderedSpace<ForceTerm>); // above the static 48 KB
+    const cudaError_t err =
+        set_smem_limit_once(reinterpret_cast<const void *>(direct_f64_kernel),
+                            static_cast<int>(smem), configured);
+    if (err != cudaSuccess) {
+        return err;
+    }
+    direct_f64_kernel<<<ceil_div(n, kOrderedTargets), OrderedShape<ForceTerm>::threads, smem,
+                        stream>>>(x, y, z, m, n, eps2, ax, ay, az);
     return cudaGetLastError();
 }
 

@@ -37,6 +37,101 @@ def test_fp64_is_bit_identical_to_reference(b200, golden_plummer):
         assert s.interaction_count().particle_particle == 2048 * 2047
 
 
+# 31-33: the edges of a chunk of sources; 16,384 and on: one target per thread.
+# The scales put squared distances below and above the range of the short
+# root and division; without softening the target's own argument is zero. (Below
+# that range, |d|^2 < 2^-895, the force's 1 / |d|^3 > 2^1342 overflows, in the
+# oracle too: opposite infinities make NaN, and only the potential is finite.)
+@pytest.mark.parametrize("n,eps,scale", [(1, 0.01, 1.0), (31, 0.0, 1.0), (32, 0.01, 1.0),
+                                         (33, 0.05, 1.0), (257, 0.0, 1e-140),
+                                         (257, 0.0, 1e137), (4097, 0.01, 1.0),
+                                         (16383, 0.01, 1.0), (16384, 0.01, 1.0),
+                                         (16415, 0.0, 1.0)])
+def test_fp64_sums_are_bit_identical_at_every_size(b200, restatement, n, eps, scale):
+    from orrery_b200 import initial_conditions as ic
+    d = ic.plummer_sphere(n, seed=n)
+    x, y, z = (d[k] * scale for k in "xyz")
+    exact, _ = restatement.direct(x, y, z, d["m"], eps)
+    a = b200.B200DirectSolver(eps, "fp64").evaluate((x, y, z), d["m"])
+    assert np.array_equal(a, exact, equal_nan=scale < 1e-100)
+    s = b200.DeviceSystem(n, eps, precision="fp64")
+    s.set_state(x, y, z, d["vx"], d["vy"], d["vz"], d["m"])
+    assert s.energy()[1] == restatement.potential_energy(x, y, z, d["m"], eps)
+
+
+def _square_roots(a, bits):
+    """Every r modulo 2^bits with r^2 = a (a = 1 modulo 8), by Hensel lifting."""
+    r = 1
+    for b in range(3, bits):
+        if (r * r - a) % (1 << (b + 1)):
+            r += 1 << (b - 1)
+    m = 1 << bits
+    return {r % m, -r % m, (r + m // 2) % m, (-r + m // 2) % m}
+
+
+# Prime factors of 2^106 - j.
+_FACTORS = {-5: [3, 7, 140627, 173331457829, 158494480927183],
+            -4: [2, 2, 257, 78919881726271091143763623681],
+            -3: [13, 6951403, 306673771, 2927433831769543],
+            -2: [2, 3, 3, 11, 43, 211, 281, 331, 5419, 86171, 664441, 1564921],
+            -1: [5, 15358129, 586477649, 1801439824104653],
+            1: [3, 107, 6361, 69431, 20394401, 28059810762433],
+            2: [2, 7, 7, 31, 71, 127, 151, 337, 29191, 106681, 122921, 152041],
+            3: [2327027, 34864072662073401681969743],
+            4: [2, 2, 3, 5, 17, 53, 157, 1613, 2731, 8191, 858001, 308761441],
+            5: [19, 29, 147240723075511219048618884109]}
+
+
+def _hard_arguments():
+    """The x whose square root, or the reciprocal of whose square root, lies so
+    near a midpoint of two doubles that a result good to 2^-103 before its last
+    rounding could round wrongly."""
+    found = []
+    # Roots: M^2 - j = x 2^k with M an odd 54-bit integer (a midpoint) and
+    # |j| <= 2 M^2 2^-103 < 64; x in [1, 2) and [2, 4) stand for every x.
+    for low, k in ((1 << 106, 54), (1 << 107, 55)):
+        for j in range(-63, 64, 8):
+            for r in _square_roots(j % (1 << k), k):
+                for odd in range(r, 1 << 54, 1 << k):
+                    square = odd * odd - j
+                    if odd >= 1 << 53 and low <= square < 2 * low and square % (1 << k) == 0:
+                        found += [np.ldexp(float(square >> k), k - 54 - 52 + 2 * e)
+                                  for e in (-420, -120, 0, 17, 350)]
+    # Reciprocals: s M = 2^106 - j with s a 53-bit integer, M a 54-bit odd one
+    # and |j| <= 2^106 2^-103.8 < 5; x = s^2, whose rounded root is s again.
+    for j, primes in _FACTORS.items():
+        n = (1 << 106) - j
+        divisors = {1}
+        for p in primes:
+            divisors |= {d * p for d in divisors}
+        assert max(divisors) == n
+        for s in divisors:
+            if 1 << 52 <= s < 1 << 53 and (n // s) % 2 == 1:
+                found += [float(np.ldexp(float(s), e - 52)) ** 2 for e in (-440, -53, 0, 1, 300)]
+    edges = [np.nextafter(4.0 ** k, 0) for k in (-200, 0, 1, 2, 300)]
+    return found + edges + [2.0 ** k for k in range(-1074, 1024, 53)]
+
+
+def test_inverse_distance_is_correctly_rounded_where_it_is_hardest(b200):
+    # Two unit masses at one point: their potential energy is minus the inverse
+    # distance of the squared softening alone.
+    import ctypes as C
+    lib = b200.load_library()
+    zero, one = np.zeros(2), np.ones(2)
+    z, m = (a.ctypes.data_as(C.POINTER(C.c_double)) for a in (zero, one))
+    arguments = _hard_arguments()
+    assert len(arguments) > 400
+    for x in arguments:
+        params = b200.make_params(b200.SOLVER_DIRECT, "fp64")
+        params.softening_squared = x
+        system, energy = C.c_void_p(), C.c_double()
+        assert lib.ob_system_create(C.byref(params), 2, C.byref(system)) == b200.OK
+        assert lib.ob_system_set_state(system, z, z, z, None, None, None, m) == b200.OK
+        assert lib.ob_system_energy(system, None, C.byref(energy)) == b200.OK
+        lib.ob_system_destroy(system)
+        assert energy.value == -(1.0 / np.sqrt(np.float64(x))), x.hex()
+
+
 def test_fp32_within_reference_bounds(b200, restatement, golden_plummer):
     g = golden_plummer
     x, y, z, m = _xyzm(g)
