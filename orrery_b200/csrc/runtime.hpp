@@ -58,6 +58,13 @@ inline cudaError_t set_smem_limit_once(const void *kernel, int bytes,
 // Sets the calling thread's last-error text and returns `code`.
 int set_error(int code, const std::string &message);
 
+// A device block of at least `bytes` on the current device: one kept from a
+// destroyed object, or newly allocated (memory.cu). Its contents are undefined.
+void *take_device_block(size_t bytes, size_t &got, int &device);
+// Keeps a block for the next object (bounded; else frees it), once the device
+// has finished what may use it.
+void keep_device_block(void *ptr, size_t bytes, int device) noexcept;
+
 // Owning device allocation that grows on demand and never shrinks, the
 // capacity policy of the reference's CUDA solvers
 // (src/solvers/cuda_direct_solver.cpp:120-137).
@@ -66,17 +73,19 @@ public:
     DeviceArray() = default;
     DeviceArray(const DeviceArray &) = delete;
     DeviceArray &operator=(const DeviceArray &) = delete;
-    DeviceArray(DeviceArray &&o) noexcept : ptr_(std::exchange(o.ptr_, nullptr)),
-                                           count_(std::exchange(o.count_, 0)) {}
+    DeviceArray(DeviceArray &&o) noexcept { swap(o); }
     DeviceArray &operator=(DeviceArray &&o) noexcept {
         if (this != &o) {
             release();
-            ptr_ = std::exchange(o.ptr_, nullptr);
-            count_ = std::exchange(o.count_, 0);
+            swap(o);
         }
         return *this;
     }
-    ~DeviceArray() { release(); }
+    ~DeviceArray() {
+        if (ptr_ != nullptr) {
+            keep_device_block(ptr_, block_bytes_, device_);
+        }
+    }
 
     // Returns true when the storage moved (callers holding the old pointer,
     // such as captured graphs, must refresh).
@@ -85,9 +94,7 @@ public:
             return false;
         }
         release();
-        void *p = nullptr;
-        check(cudaMalloc(&p, count * sizeof(T)), "device allocation");
-        ptr_ = static_cast<T *>(p);
+        ptr_ = static_cast<T *>(take_device_block(count * sizeof(T), block_bytes_, device_));
         count_ = count;
         return true;
     }
@@ -103,8 +110,17 @@ public:
     [[nodiscard]] size_t bytes() const noexcept { return count_ * sizeof(T); }
 
 private:
+    void swap(DeviceArray &o) noexcept {
+        std::swap(ptr_, o.ptr_);
+        std::swap(count_, o.count_);
+        std::swap(block_bytes_, o.block_bytes_);
+        std::swap(device_, o.device_);
+    }
+
     T *ptr_ = nullptr;
     size_t count_ = 0;
+    size_t block_bytes_ = 0; // of the whole block, which may exceed count_ values
+    int device_ = 0;
 };
 
 // Records `event` on `stream`; `external` makes it a real event-record node

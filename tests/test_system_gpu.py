@@ -303,3 +303,39 @@ def test_the_symmetric_methods_run_backwards_to_where_they_started(b200, integra
         for keys in (("x", "y", "z"), ("vx", "vy", "vz")):
             error = np.linalg.norm([end[k][i] - start[k][i] for k in keys])
             assert error <= tolerance, (i, keys, error)
+
+
+def test_blocks_of_destroyed_objects_serve_new_ones_from_several_threads(b200, restatement):
+    # Solvers and systems made and dropped in four threads, their device blocks
+    # passing from one to the next: every result stays the oracle's bit for bit.
+    import threading
+
+    from orrery_b200 import initial_conditions as ic
+    sizes = [33, 700, 1500, 2049]
+    data = {n: ic.plummer_sphere(n, seed=n) for n in sizes}
+    want = {n: (restatement.direct(d["x"], d["y"], d["z"], d["m"], 0.01)[0],
+                restatement.barnes_hut(d["x"], d["y"], d["z"], d["m"], 0.02, 0.7, 8, True)[0])
+            for n, d in data.items()}
+    failures = []
+
+    def work(offset):
+        for k in range(12):
+            n = sizes[(k + offset) % len(sizes)]
+            d = data[n]
+            xyz, direct, tree = (d["x"], d["y"], d["z"]), *want[n]
+            got = b200.B200DirectSolver(0.01, "fp64").evaluate(xyz, d["m"])
+            got_tree = b200.B200TreeSolver(0.02, 0.7, 8, True, "fp64").evaluate(xyz, d["m"])
+            s = b200.DeviceSystem(n, 0.01, precision="fp64")
+            s.set_state(*xyz, d["vx"], d["vy"], d["vz"], d["m"])
+            st = s.state()
+            field = np.stack([st["ax"], st["ay"], st["az"]], axis=1)
+            if not (np.array_equal(got, direct) and np.array_equal(got_tree, tree) and
+                    np.array_equal(field, direct)):
+                failures.append((offset, k, n))
+
+    threads = [threading.Thread(target=work, args=(t,)) for t in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not failures
