@@ -19,11 +19,15 @@
 //     the zero-mass padding add exactly zero (self_term_vanishes), and
 //     without it the tiles that hold them select zero mass for j == i and
 //     j >= n, as the reference kernel masks (cuda_direct_kernel.cu:155-160);
-//   * when the targets alone cannot fill 148 SMs, S CTAs of one thread-block
-//     cluster split the source range and their partial sums are reduced through
-//     distributed shared memory in a fixed rank order (deterministic).
+//   * when the targets alone cannot fill 148 SMs evenly, S CTAs split the source
+//     range of a target tile. Where the whole grid is resident at once they form
+//     a thread-block cluster, whose partial sums are reduced through distributed
+//     shared memory; otherwise each leaves its sums in memory and the last to
+//     arrive adds them (a cluster waits for as many free slots of one GPC as it
+//     has CTAs, which idles SMs once slots free up one by one). Either way the
+//     parts are added in order, so the result does not depend on scheduling.
+#include <algorithm>
 #include <cooperative_groups.h>
-#include <type_traits>
 
 #include "common.cuh"
 #include "f64_math.cuh"
@@ -47,6 +51,8 @@ struct DirectArgs {
     double *ay;
     double *az;
     unsigned *status;
+    double *partial;   // sums of the parts (a part is its own CTA, no cluster), or NULL
+    unsigned *arrived; // per target tile: parts that have written theirs (zero between launches)
 };
 
 // Range of source tiles [tb, te) handled by split rank `rank`.
@@ -62,6 +68,13 @@ __device__ __forceinline__ void source_tiles(uint32_t n, uint32_t split, uint32_
 // pair (the shapes for small systems, few warps per SM) gets more independent
 // chains to overlap.
 template <int P> constexpr int kSourceUnroll = P == 1 ? 4 : 2;
+
+// The same for the FP32 kernel, in pairs of sources per step.
+template <int R> constexpr int kPairUnroll = R == 2 ? 4 : 2;
+// Threads per SM that the FP32 kernel's registers are held to: 512 at 128
+// registers with four targets and more (262,144 targets 26.8 ms; 768 at 80
+// 27.4 ms, 1024 at 64 30.2 ms), 1024 at 64 with two.
+template <int THREADS, int R> constexpr int kMinBlocksF32 = (R <= 2 ? 1024 : 512) / THREADS;
 
 // Tiles holding the CTA's own targets or padding need no masks when those
 // entries add exactly zero. A target's own entry is its packed position, so
@@ -86,15 +99,73 @@ template <int THREADS, int K> struct SourceGroups {
     static constexpr uint32_t sources = kDirectTile / K; // sources per slice of a tile
 };
 
-// Shared-memory type of the CTA's per-target sums: FP32 sums pass through
-// exactly as float when a CTA has one group; group sums are FP64.
-template <int K, typename T> using PartialType = std::conditional_t<K == 1, T, double>;
 
-// Writes the CTA's per-target sums, reducing across the cluster when split.
-// `partial` holds 3*BT values of type T laid out [component][slot] (K*3*BT
-// doubles, one block per group, when K > 1). Target slot r*TP + lane.
-template <int THREADS, int R, int K, typename T>
-__device__ __forceinline__ void finish_targets(const DirectArgs &a, uint32_t t0, T *partial,
+// Adds the parts of a CTA's target tile, whose 3 * bt sums ([component][slot])
+// this part holds in shared memory. Kept out of line: inlined, it changes the
+// registers the compiler gives the pair loops.
+__device__ __noinline__ void add_parts(const DirectArgs &a, uint32_t t0, double *partial,
+                                       uint32_t bt) {
+    const uint32_t split = gridDim.x, rank = blockIdx.x, tid = threadIdx.x;
+    const uint32_t block = 3u * bt; // one part's sums
+    if (a.partial != nullptr) {
+        __shared__ bool last;
+        __syncthreads();
+        double *sums = a.partial + static_cast<size_t>(blockIdx.y) * split * block;
+        for (uint32_t k = tid; k < block; k += blockDim.x) {
+            sums[rank * block + k] = partial[k];
+        }
+        __threadfence();
+        __syncthreads();
+        if (tid == 0) {
+            last = atomicAdd(&a.arrived[blockIdx.y], 1u) == split - 1u;
+        }
+        __syncthreads();
+        if (!last) {
+            return;
+        }
+        __threadfence();
+        for (uint32_t k = tid; k < block; k += blockDim.x) {
+            double sum = 0.0;
+            for (uint32_t q = 0; q < split; ++q) {
+                sum += __ldcg(&sums[q * block + k]);
+            }
+            const uint32_t i = t0 + k % bt;
+            if (i < a.n) {
+                (k < bt ? a.ax : k < 2u * bt ? a.ay : a.az)[i] = sum;
+            }
+        }
+        if (tid == 0) {
+            a.arrived[blockIdx.y] = 0u; // for the next launch
+        }
+        return;
+    }
+    cg::cluster_group cluster = cg::this_cluster();
+    cluster.sync();
+    const uint32_t per = bt / split;
+    for (uint32_t k = tid; k < per; k += blockDim.x) {
+        const uint32_t slot = rank * per + k;
+        double s0 = 0.0, s1 = 0.0, s2 = 0.0;
+        for (uint32_t q = 0; q < split; ++q) {
+            const double *remote = cluster.map_shared_rank(partial, q);
+            s0 += remote[slot];
+            s1 += remote[bt + slot];
+            s2 += remote[2 * bt + slot];
+        }
+        const uint32_t i = t0 + slot;
+        if (i < a.n) {
+            a.ax[i] = s0;
+            a.ay[i] = s1;
+            a.az[i] = s2;
+        }
+    }
+    cluster.sync();
+}
+
+// Writes the CTA's per-target sums, adding the parts' when the sources are
+// split. `partial` holds 3*BT sums laid out [component][slot] (one such block
+// per group). Target slot r*TP + lane.
+template <int THREADS, int R, int K>
+__device__ __forceinline__ void finish_targets(const DirectArgs &a, uint32_t t0, double *partial,
                                                const double (&sx)[R], const double (&sy)[R],
                                                const double (&sz)[R]) {
     constexpr uint32_t TP = SourceGroups<THREADS, K>::lanes;
@@ -119,12 +190,11 @@ __device__ __forceinline__ void finish_targets(const DirectArgs &a, uint32_t t0,
 #pragma unroll
         for (int r = 0; r < R; ++r) {
             const uint32_t slot = r * THREADS + tid;
-            partial[slot] = static_cast<T>(sx[r]);
-            partial[BT + slot] = static_cast<T>(sy[r]);
-            partial[2 * BT + slot] = static_cast<T>(sz[r]);
+            partial[slot] = sx[r];
+            partial[BT + slot] = sy[r];
+            partial[2 * BT + slot] = sz[r];
         }
     } else {
-        static_assert(sizeof(T) == sizeof(double), "group sums are FP64");
         // Each group's sums in its own block, then added in group order into
         // block 0 (each slot by one thread, which reads every group's value of
         // a component before it overwrites block 0's).
@@ -160,69 +230,49 @@ __device__ __forceinline__ void finish_targets(const DirectArgs &a, uint32_t t0,
             return;
         }
     }
-    cg::cluster_group cluster = cg::this_cluster();
-    cluster.sync();
-    const uint32_t rank = blockIdx.x;
-    const uint32_t per = BT / split;
-    for (uint32_t k = tid; k < per; k += THREADS) {
-        const uint32_t slot = rank * per + k;
-        double s0 = 0.0, s1 = 0.0, s2 = 0.0;
-        for (uint32_t q = 0; q < split; ++q) {
-            const T *remote = cluster.map_shared_rank(partial, q);
-            s0 += static_cast<double>(remote[slot]);
-            s1 += static_cast<double>(remote[BT + slot]);
-            s2 += static_cast<double>(remote[2 * BT + slot]);
-        }
-        const uint32_t i = t0 + slot;
-        if (i < a.n) {
-            a.ax[i] = s0;
-            a.ay[i] = s1;
-            a.az[i] = s2;
-        }
-    }
-    cluster.sync();
+    add_parts(a, t0, partial, BT);
 }
 
-// Sources of the FP32 kernel are stored pre-duplicated, two float4 per
-// particle: (x, x, y, y) and (z, z, m, m), so that each half is already a
-// packed FP32x2 operand for a pair of targets and no register moves are needed.
+// Sources of the FP32 kernel are stored in pairs, two float4 per two
+// particles: (x0, x1, y0, y1) and (z0, z1, m0, m1), so that each half is already
+// a packed FP32x2 operand of two sources; a target's coordinates are held
+// twice in registers. (With the values duplicated in memory and pairs of
+// targets per instruction, a warp read twice the shared memory per
+// interaction, two thirds of what the SM can deliver to four-target threads:
+// 262,144 targets took 29.2 ms.)
 template <int THREADS, int R, int K>
-__global__ void __launch_bounds__(THREADS) direct_f32_kernel(const DirectArgs a) {
-    static_assert(R % 2 == 0, "targets are processed in packed pairs");
-    constexpr int P = R / 2;
+__global__ void __launch_bounds__(THREADS, kMinBlocksF32<THREADS, R>)
+    direct_f32_kernel(const DirectArgs a) {
     extern __shared__ __align__(128) unsigned char smem[];
     constexpr uint32_t TP = SourceGroups<THREADS, K>::lanes;
     constexpr uint32_t JS = SourceGroups<THREADS, K>::sources;
     constexpr uint32_t BT = TP * R;
-    using PT = PartialType<K, float>;
-    float4 *tiles = reinterpret_cast<float4 *>(smem); // 2 buffers x 2*kDirectTile
-    uint64_t *bars = reinterpret_cast<uint64_t *>(smem + 4 * kDirectTile * sizeof(float4));
-    PT *partial = reinterpret_cast<PT *>(bars + 2);
+    float4 *tiles = reinterpret_cast<float4 *>(smem); // 2 buffers x kDirectTile
+    uint64_t *bars = reinterpret_cast<uint64_t *>(smem + 2 * kDirectTile * sizeof(float4));
+    double *partial = reinterpret_cast<double *>(bars + 2);
 
     const uint32_t tid = threadIdx.x;
     const uint32_t lane = tid % TP;
-    const uint32_t jb = (tid / TP) * JS; // this thread's slice of every tile
+    const uint32_t pb = (tid / TP) * (JS / 2); // this thread's slice of every tile, in pairs
     const uint32_t t0 = blockIdx.y * BT;
     const float2 eps2 = make_float2(a.eps2, a.eps2);
 
-    // Target r = 2p + h is slot (2p + h) * TP + lane; pair p packs h = 0, 1.
-    float2 nx[P], ny[P], nz[P], ax[P], ay[P], az[P];
+    // Target r is slot r * TP + lane.
+    float2 nx[R], ny[R], nz[R], ax[R], ay[R], az[R];
     const float y_self = rsqrt_approx(a.eps2);
     bool vanish = true;
 #pragma unroll
-    for (int p = 0; p < P; ++p) {
-        const float4 u0 = a.hi[2ull * (t0 + (2 * p) * TP + lane)];
-        const float4 u1 = a.hi[2ull * (t0 + (2 * p) * TP + lane) + 1];
-        const float4 v0 = a.hi[2ull * (t0 + (2 * p + 1) * TP + lane)];
-        const float4 v1 = a.hi[2ull * (t0 + (2 * p + 1) * TP + lane) + 1];
-        nx[p] = make_float2(-u0.x, -v0.x);
-        ny[p] = make_float2(-u0.z, -v0.z);
-        nz[p] = make_float2(-u1.x, -v1.x);
-        ax[p] = ay[p] = az[p] = make_float2(0.0f, 0.0f);
-        const float2 ys = make_float2(y_self, y_self);
-        const float2 f_self = __fmul2_rn(__fmul2_rn(make_float2(u1.z, v1.z), ys), __fmul2_rn(ys, ys));
-        vanish = vanish && self_term_vanishes(a.eps2, f_self.x) &&
-                 self_term_vanishes(a.eps2, f_self.y);
+    for (int r = 0; r < R; ++r) {
+        const uint32_t i = t0 + r * TP + lane;
+        const float4 u0 = a.hi[i & ~1u], u1 = a.hi[i | 1u];
+        const bool odd = (i & 1u) != 0u;
+        const float x = odd ? u0.y : u0.x, y = odd ? u0.w : u0.z, z = odd ? u1.y : u1.x;
+        const float m = odd ? u1.w : u1.z;
+        nx[r] = make_float2(-x, -x);
+        ny[r] = make_float2(-y, -y);
+        nz[r] = make_float2(-z, -z);
+        ax[r] = ay[r] = az[r] = make_float2(0.0f, 0.0f);
+        vanish = vanish && self_term_vanishes(a.eps2, (m * y_self) * (y_self * y_self));
     }
 
     uint32_t tb, te;
@@ -233,11 +283,11 @@ __global__ void __launch_bounds__(THREADS) direct_f32_kernel(const DirectArgs a)
         fence_barrier_init();
     }
     const bool unmasked = __syncthreads_and(vanish ? 1 : 0) != 0;
-    constexpr uint32_t tile_bytes = 2 * kDirectTile * sizeof(float4);
+    constexpr uint32_t tile_bytes = kDirectTile * sizeof(float4);
     auto stage = [&](uint32_t k, uint32_t buf) {
         mbar_arrive_expect_tx(&bars[buf], tile_bytes);
-        bulk_copy_g2s(tiles + buf * 2 * kDirectTile,
-                      a.hi + 2ull * static_cast<size_t>(k) * kDirectTile, tile_bytes, &bars[buf]);
+        bulk_copy_g2s(tiles + buf * kDirectTile, a.hi + static_cast<size_t>(k) * kDirectTile,
+                      tile_bytes, &bars[buf]);
     };
     if (tid == 0) {
         for (uint32_t k = tb; k < min(tb + 2, te); ++k) {
@@ -253,48 +303,47 @@ __global__ void __launch_bounds__(THREADS) direct_f32_kernel(const DirectArgs a)
             ok = mbar_wait_bounded(&bars[buf], (it >> 1) & 1u, a.status);
         }
         if (ok) {
-            const float4 *tile = tiles + buf * 2 * kDirectTile;
+            const float4 *tile = tiles + buf * kDirectTile;
             const uint32_t j0 = k * kDirectTile;
             const bool masked = !unmasked && ((j0 + kDirectTile > a.n) ||
                                               (j0 < t0 + BT && t0 < j0 + kDirectTile));
             if (!masked) {
-#pragma unroll(kSourceUnroll<P>)
-                for (uint32_t jj = jb; jj < jb + JS; ++jj) {
-                    const float4 s0 = tile[2 * jj];     // (x, x, y, y)
-                    const float4 s1 = tile[2 * jj + 1]; // (z, z, m, m)
+#pragma unroll(kPairUnroll<R>)
+                for (uint32_t p = pb; p < pb + JS / 2; ++p) {
+                    const float4 s0 = tile[2 * p];     // (x0, x1, y0, y1)
+                    const float4 s1 = tile[2 * p + 1]; // (z0, z1, m0, m1)
                     const float2 sx = make_float2(s0.x, s0.y);
                     const float2 sy = make_float2(s0.z, s0.w);
                     const float2 sz = make_float2(s1.x, s1.y);
                     const float2 sm = make_float2(s1.z, s1.w);
 #pragma unroll
-                    for (int p = 0; p < P; ++p) {
-                        const float2 dx = __fadd2_rn(sx, nx[p]);
-                        const float2 dy = __fadd2_rn(sy, ny[p]);
-                        const float2 dz = __fadd2_rn(sz, nz[p]);
+                    for (int r = 0; r < R; ++r) {
+                        const float2 dx = __fadd2_rn(sx, nx[r]);
+                        const float2 dy = __fadd2_rn(sy, ny[r]);
+                        const float2 dz = __fadd2_rn(sz, nz[r]);
                         float2 r2 = __ffma2_rn(dx, dx, eps2);
                         r2 = __ffma2_rn(dy, dy, r2);
                         r2 = __ffma2_rn(dz, dz, r2);
                         const float2 inv = make_float2(rsqrt_approx(r2.x), rsqrt_approx(r2.y));
                         const float2 f = __fmul2_rn(__fmul2_rn(sm, inv), __fmul2_rn(inv, inv));
-                        ax[p] = __ffma2_rn(f, dx, ax[p]);
-                        ay[p] = __ffma2_rn(f, dy, ay[p]);
-                        az[p] = __ffma2_rn(f, dz, az[p]);
+                        ax[r] = __ffma2_rn(f, dx, ax[r]);
+                        ay[r] = __ffma2_rn(f, dy, ay[r]);
+                        az[r] = __ffma2_rn(f, dz, az[r]);
                     }
                 }
             } else {
-                for (uint32_t jj = jb; jj < jb + JS; ++jj) {
-                    const float4 s0 = tile[2 * jj];
-                    const float4 s1 = tile[2 * jj + 1];
-                    const uint32_t j = j0 + jj;
+                for (uint32_t p = pb; p < pb + JS / 2; ++p) {
+                    const float4 s0 = tile[2 * p];
+                    const float4 s1 = tile[2 * p + 1];
+                    const uint32_t j = j0 + 2 * p;
 #pragma unroll
-                    for (int p = 0; p < P; ++p) {
-                        const uint32_t i0 = t0 + (2 * p) * TP + lane;
-                        const uint32_t i1 = i0 + TP;
-                        const bool skip0 = (j == i0) || (j >= a.n);
-                        const bool skip1 = (j == i1) || (j >= a.n);
-                        const float2 dx = __fadd2_rn(make_float2(s0.x, s0.y), nx[p]);
-                        const float2 dy = __fadd2_rn(make_float2(s0.z, s0.w), ny[p]);
-                        const float2 dz = __fadd2_rn(make_float2(s1.x, s1.y), nz[p]);
+                    for (int r = 0; r < R; ++r) {
+                        const uint32_t i = t0 + r * TP + lane;
+                        const bool skip0 = (j == i) || (j >= a.n);
+                        const bool skip1 = (j + 1 == i) || (j + 1 >= a.n);
+                        const float2 dx = __fadd2_rn(make_float2(s0.x, s0.y), nx[r]);
+                        const float2 dy = __fadd2_rn(make_float2(s0.z, s0.w), ny[r]);
+                        const float2 dz = __fadd2_rn(make_float2(s1.x, s1.y), nz[r]);
                         float2 r2 = __ffma2_rn(dx, dx, eps2);
                         r2 = __ffma2_rn(dy, dy, r2);
                         r2 = __ffma2_rn(dz, dz, r2);
@@ -303,9 +352,9 @@ __global__ void __launch_bounds__(THREADS) direct_f32_kernel(const DirectArgs a)
                         const float2 w = make_float2(skip0 ? 0.0f : s1.z, skip1 ? 0.0f : s1.w);
                         const float2 inv = make_float2(rsqrt_approx(r2.x), rsqrt_approx(r2.y));
                         const float2 f = __fmul2_rn(__fmul2_rn(w, inv), __fmul2_rn(inv, inv));
-                        ax[p] = __ffma2_rn(f, dx, ax[p]);
-                        ay[p] = __ffma2_rn(f, dy, ay[p]);
-                        az[p] = __ffma2_rn(f, dz, az[p]);
+                        ax[r] = __ffma2_rn(f, dx, ax[r]);
+                        ay[r] = __ffma2_rn(f, dy, ay[r]);
+                        az[r] = __ffma2_rn(f, dz, az[r]);
                     }
                 }
             }
@@ -319,15 +368,12 @@ __global__ void __launch_bounds__(THREADS) direct_f32_kernel(const DirectArgs a)
 
     double sx[R], sy[R], sz[R];
 #pragma unroll
-    for (int p = 0; p < P; ++p) {
-        sx[2 * p] = ax[p].x;
-        sx[2 * p + 1] = ax[p].y;
-        sy[2 * p] = ay[p].x;
-        sy[2 * p + 1] = ay[p].y;
-        sz[2 * p] = az[p].x;
-        sz[2 * p + 1] = az[p].y;
+    for (int r = 0; r < R; ++r) {
+        sx[r] = static_cast<double>(ax[r].x) + static_cast<double>(ax[r].y);
+        sy[r] = static_cast<double>(ay[r].x) + static_cast<double>(ay[r].y);
+        sz[r] = static_cast<double>(az[r].x) + static_cast<double>(az[r].y);
     }
-    finish_targets<THREADS, R, K, PT>(a, t0, partial, sx, sy, sz);
+    finish_targets<THREADS, R, K>(a, t0, partial, sx, sy, sz);
 }
 
 // Split (precision) form: targets r = 2p + h are packed in pairs p and every
@@ -468,7 +514,7 @@ __global__ void __launch_bounds__(THREADS) direct_split_kernel(const DirectArgs 
             stage(k + 2, buf);
         }
     }
-    finish_targets<THREADS, R, K, double>(a, t0, partial, sx, sy, sz);
+    finish_targets<THREADS, R, K>(a, t0, partial, sx, sy, sz);
 }
 
 // FP64 direct sum in the order of accumulate_range_scalar
@@ -644,12 +690,12 @@ __global__ void __launch_bounds__(kWideThreads)
     }
 }
 
-// Packs FP64 SoA into the kernels' source layout: two float4 per particle,
-// (x, x, y, y) and (z, z, m, m) rounded to FP32, and in the split form (lo
-// given) two more, (x', x', y', y') and (z', z', 0, 0) with x' = x - FP32(x).
-__global__ void pack_kernel(const double *__restrict__ x, const double *__restrict__ y,
-                            const double *__restrict__ z, const double *__restrict__ m,
-                            uint32_t n, uint32_t padded, float4 *hi, float4 *lo) {
+// Packs FP64 SoA into the split form's source layout: two float4 per particle,
+// (x, x, y, y) and (z, z, m, m) rounded to FP32 in hi, and (x', x', y', y') and
+// (z', z', 0, 0) with x' = x - FP32(x) in lo.
+__global__ void pack_split_kernel(const double *__restrict__ x, const double *__restrict__ y,
+                                  const double *__restrict__ z, const double *__restrict__ m,
+                                  uint32_t n, uint32_t padded, float4 *hi, float4 *lo) {
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < padded;
          i += gridDim.x * blockDim.x) {
         const bool real = i < n;
@@ -660,22 +706,38 @@ __global__ void pack_kernel(const double *__restrict__ x, const double *__restri
         const float hm = real ? __double2float_rn(m[i]) : 0.0f;
         hi[2ull * i] = make_float4(hx, hx, hy, hy);
         hi[2ull * i + 1] = make_float4(hz, hz, hm, hm);
-        if (lo != nullptr) {
-            // X - hx is exact in FP64; rounding it gives the low part.
-            const float lx = __double2float_rn(X - static_cast<double>(hx));
-            const float ly = __double2float_rn(Y - static_cast<double>(hy));
-            const float lz = __double2float_rn(Z - static_cast<double>(hz));
-            lo[2ull * i] = make_float4(lx, lx, ly, ly);
-            lo[2ull * i + 1] = make_float4(lz, lz, 0.0f, 0.0f);
-        }
+        // X - hx is exact in FP64; rounding it gives the low part.
+        const float lx = __double2float_rn(X - static_cast<double>(hx));
+        const float ly = __double2float_rn(Y - static_cast<double>(hy));
+        const float lz = __double2float_rn(Z - static_cast<double>(hz));
+        lo[2ull * i] = make_float4(lx, lx, ly, ly);
+        lo[2ull * i + 1] = make_float4(lz, lz, 0.0f, 0.0f);
+    }
+}
+
+// Packs FP64 SoA into the FP32 kernel's pairs, two float4 per two particles:
+// (x0, x1, y0, y1) and (z0, z1, m0, m1); `padded` is even.
+__global__ void pack_pairs_kernel(const double *__restrict__ x, const double *__restrict__ y,
+                                  const double *__restrict__ z, const double *__restrict__ m,
+                                  uint32_t n, uint32_t padded, float4 *pairs) {
+    for (uint32_t i = 2u * (blockIdx.x * blockDim.x + threadIdx.x); i < padded;
+         i += 2u * gridDim.x * blockDim.x) {
+        const bool a = i < n, b = i + 1u < n;
+        pairs[i] = make_float4(a ? __double2float_rn(x[i]) : 0.0f,
+                               b ? __double2float_rn(x[i + 1u]) : 0.0f,
+                               a ? __double2float_rn(y[i]) : 0.0f,
+                               b ? __double2float_rn(y[i + 1u]) : 0.0f);
+        pairs[i + 1u] = make_float4(a ? __double2float_rn(z[i]) : 0.0f,
+                                    b ? __double2float_rn(z[i + 1u]) : 0.0f,
+                                    a ? __double2float_rn(m[i]) : 0.0f,
+                                    b ? __double2float_rn(m[i + 1u]) : 0.0f);
     }
 }
 
 template <int THREADS, int R, int K, bool SPLIT> size_t direct_smem_bytes() {
-    const size_t tiles = (SPLIT ? 8 : 4) * kDirectTile * sizeof(float4);
+    const size_t tiles = (SPLIT ? 8 : 2) * kDirectTile * sizeof(float4);
     // 3 sums per target: THREADS * R / K targets, one block per group.
-    const size_t partial =
-        3 * THREADS * R * (SPLIT ? sizeof(double) : sizeof(PartialType<K, float>));
+    const size_t partial = 3 * THREADS * R * sizeof(double);
     return tiles + 2 * sizeof(uint64_t) + partial;
 }
 
@@ -708,7 +770,7 @@ cudaError_t launch_direct_t(const DirectArgs &args, int split, cudaStream_t stre
     cfg.stream = stream;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = static_cast<unsigned>(split);
+    attr[0].val.clusterDim.x = args.partial != nullptr ? 1u : static_cast<unsigned>(split);
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
@@ -741,13 +803,34 @@ cudaError_t dispatch_direct(const DirectArgs &args, const DirectConfig &c, cudaS
     return cudaErrorInvalidValue;
 }
 
-bool valid_split(int split) { return split == 1 || split == 2 || split == 4 || split == 8; }
+uint32_t targets_per_cta(const DirectConfig &c) {
+    return static_cast<uint32_t>(c.threads * c.targets_per_thread / c.groups);
+}
 
 } // namespace
 
+bool direct_uses_cluster(uint32_t n, const DirectConfig &c) {
+    // The grid fits the SMs at two CTAs each, and the parts a portable cluster.
+    const bool portable = c.split == 1 || c.split == 2 || c.split == 4 || c.split == 8;
+    return portable && (c.split == 1 || static_cast<uint64_t>(ceil_div(n, targets_per_cta(c))) *
+                                                static_cast<uint64_t>(c.split) <=
+                                            2u * 148u);
+}
+
+size_t direct_partial_doubles(uint32_t n, const DirectConfig &c) {
+    if (direct_uses_cluster(n, c)) {
+        return 0;
+    }
+    const uint32_t bt = targets_per_cta(c);
+    return 3ull * bt * ceil_div(n, bt) * static_cast<size_t>(c.split);
+}
+
+size_t direct_arrival_words(uint32_t n, const DirectConfig &c) {
+    return direct_uses_cluster(n, c) ? 0 : ceil_div(n, targets_per_cta(c));
+}
+
 uint32_t direct_padded_count(uint32_t n, const DirectConfig &config) {
-    const uint32_t bt =
-        static_cast<uint32_t>(config.threads * config.targets_per_thread / config.groups);
+    const uint32_t bt = targets_per_cta(config);
     const uint32_t unit = bt > kDirectTile ? bt : kDirectTile;
     const uint32_t padded = ceil_div(n, unit) * unit;
     return padded == 0 ? unit : padded;
@@ -760,35 +843,46 @@ cudaError_t pack_sources(const double *x, const double *y, const double *z, cons
         return cudaSuccess;
     }
     const uint32_t threads = 256;
-    const uint32_t blocks = min(ceil_div(padded, threads), 148u * 16u);
-    pack_kernel<<<blocks, threads, 0, stream>>>(x, y, z, m, n, padded, hi, lo);
+    if (lo != nullptr) {
+        const uint32_t blocks = min(ceil_div(padded, threads), 148u * 16u);
+        pack_split_kernel<<<blocks, threads, 0, stream>>>(x, y, z, m, n, padded, hi, lo);
+    } else {
+        const uint32_t blocks = min(ceil_div(padded / 2u, threads), 148u * 16u);
+        pack_pairs_kernel<<<blocks, threads, 0, stream>>>(x, y, z, m, n, padded, hi);
+    }
     return cudaGetLastError();
 }
 
 cudaError_t launch_direct_f32(const float4 *sources, uint32_t n, uint32_t padded, float eps2,
                               double *ax, double *ay, double *az, const DirectConfig &config,
-                              unsigned *status, cudaStream_t stream) {
+                              const DirectParts &parts, unsigned *status, cudaStream_t stream) {
     if (n == 0) {
         return cudaSuccess;
     }
-    if (!valid_split(config.split) || padded < direct_padded_count(n, config)) {
+    const bool cluster = direct_uses_cluster(n, config);
+    if (config.split < 1 || padded < direct_padded_count(n, config) ||
+        (!cluster && (parts.sums == nullptr || parts.arrived == nullptr))) {
         return cudaErrorInvalidValue;
     }
-    const DirectArgs args{sources, nullptr, n, padded, eps2, ax, ay, az, status};
+    const DirectArgs args{sources, nullptr, n, padded, eps2, ax, ay, az, status,
+                          cluster ? nullptr : parts.sums, parts.arrived};
     return dispatch_direct<false>(args, config, stream);
 }
 
 cudaError_t launch_direct_split(const float4 *hi, const float4 *lo, uint32_t n, uint32_t padded,
                                 float eps2, double *ax, double *ay, double *az,
-                                const DirectConfig &config, unsigned *status,
-                                cudaStream_t stream) {
+                                const DirectConfig &config, const DirectParts &parts,
+                                unsigned *status, cudaStream_t stream) {
     if (n == 0) {
         return cudaSuccess;
     }
-    if (!valid_split(config.split) || padded < direct_padded_count(n, config)) {
+    const bool cluster = direct_uses_cluster(n, config);
+    if (config.split < 1 || padded < direct_padded_count(n, config) ||
+        (!cluster && (parts.sums == nullptr || parts.arrived == nullptr))) {
         return cudaErrorInvalidValue;
     }
-    const DirectArgs args{hi, lo, n, padded, eps2, ax, ay, az, status};
+    const DirectArgs args{hi, lo, n, padded, eps2, ax, ay, az, status,
+                          cluster ? nullptr : parts.sums, parts.arrived};
     return dispatch_direct<true>(args, config, stream);
 }
 
@@ -842,25 +936,64 @@ int direct_candidates(bool split, DirectConfig *out, int capacity) {
     return count;
 }
 
-DirectConfig direct_default_config(uint32_t n, bool split, int sm_count) {
-    // The pattern of the shapes the autotuner picks on B200 from 1,000 to
-    // 262,144 particles: 256-thread CTAs in source groups of one warp (of two
-    // for the split form's four-target threads, whose registers allow fewer
-    // warps), two targets per thread for small systems and four from 8192 on,
-    // and the sources split across a cluster until about four CTAs per SM.
-    const uint32_t sms = static_cast<uint32_t>(sm_count > 0 ? sm_count : 148);
-    DirectConfig c;
-    c.threads = 256;
-    c.targets_per_thread = n >= 8192u ? 4 : 2;
-    c.groups = split && c.targets_per_thread == 4 ? 4 : 8;
-    const uint32_t bt = static_cast<uint32_t>(c.threads * c.targets_per_thread / c.groups);
-    const uint32_t blocks = ceil_div(n, bt);
+// Estimated time of a shape, in units of one target against one tile of
+// sources on one SM: the CTAs that an SM gets (half a one more than the mean,
+// for the uneven end, where an SM is left with one of its two), times a CTA's
+// work and its start and end, times what the shape costs per pair beside
+// the cheapest one.
+static double direct_cost(const DirectConfig &c, double per_pair, uint32_t n, uint32_t sms) {
+    const uint32_t bt = targets_per_cta(c);
     const uint32_t tiles = ceil_div(n, kDirectTile);
-    while (c.split < 8 && blocks * static_cast<uint32_t>(c.split) < 4u * sms &&
-           static_cast<uint32_t>(c.split * 2) <= tiles) {
-        c.split *= 2;
+    const auto parts = static_cast<uint32_t>(c.split);
+    const uint64_t ctas = static_cast<uint64_t>(ceil_div(n, bt)) * parts;
+    const bool alone = ctas <= sms; // one CTA per SM at most
+    const double per_sm =
+        alone ? 1.0 : ctas <= 2ull * sms ? 2.0 : static_cast<double>(ctas) / sms + 0.5;
+    double cost = per_pair * per_sm * bt * (ceil_div(tiles, parts) + 0.15);
+    if (alone) { // a CTA alone on its SM hides less latency
+        cost /= c.targets_per_thread == 2 ? 0.83 : 0.95;
     }
-    return c;
+    return cost;
+}
+
+DirectConfig direct_default_config(uint32_t n, bool split, int sm_count) {
+    // The cheapest of a few 256-thread shapes by the estimate above, whose
+    // constants are fitted to sweeps from 1,000 to 262,144 particles on B200.
+    // What decides is how evenly the CTAs fill the SMs: with one cluster rule
+    // for all sizes (parts until about four CTAs per SM) FP32 sums of 20,011,
+    // 40,000 and 65,536 particles took 222, 862 and 1,931 us, now 179, 674 and
+    // 1,737; split sums of 10,007 and 65,536 178 us and 5.0 ms, now 127 us and
+    // 4.2 ms.
+    const uint32_t sms = static_cast<uint32_t>(sm_count > 0 ? sm_count : 148);
+    struct Shape {
+        int targets, groups;
+        double per_pair;
+    };
+    static const Shape fp32_shapes[] = {{4, 8, 1.0}, {2, 8, 1.01}};
+    static const Shape split_shapes[] = {{4, 8, 1.0}, {4, 4, 0.985}, {2, 8, 1.06}};
+    static const int parts_tried[] = {1, 2, 4, 8, 3, 5, 6, 10, 12, 16, 24, 32};
+    const Shape *shapes = split ? split_shapes : fp32_shapes;
+    const int shape_count = split ? 3 : 2;
+    DirectConfig best;
+    double best_cost = 0.0;
+    for (int k = 0; k < shape_count; ++k) {
+        for (const int parts : parts_tried) {
+            if (parts > 1 && static_cast<uint32_t>(parts) > ceil_div(n, kDirectTile)) {
+                continue;
+            }
+            DirectConfig c;
+            c.threads = 256;
+            c.targets_per_thread = shapes[k].targets;
+            c.groups = shapes[k].groups;
+            c.split = parts;
+            const double cost = direct_cost(c, shapes[k].per_pair, n, sms);
+            if (best_cost == 0.0 || cost < best_cost) {
+                best = c;
+                best_cost = cost;
+            }
+        }
+    }
+    return best;
 }
 
 } // namespace ob

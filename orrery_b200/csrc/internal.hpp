@@ -9,8 +9,8 @@
 namespace ob {
 
 // Tile shape of the direct kernels: THREADS threads per CTA, R targets per
-// thread, and S CTAs (one thread-block cluster) splitting the source range of
-// one target tile. Chosen by the autotuner (direct_config_for).
+// thread, and S CTAs (parts) splitting the source range of one target tile.
+// direct_default_config's pick, or the autotuner's.
 struct DirectConfig {
     int threads = 256;
     int targets_per_thread = 4;
@@ -25,17 +25,30 @@ constexpr uint32_t kDirectTile = 512;
 uint32_t direct_padded_count(uint32_t n, const DirectConfig &config);
 
 // Packs FP64 SoA into the direct kernels' source layout, zero-padded to
-// `padded` particles. FP32 form (lo == nullptr): 2 * padded float4 in `hi`,
-// (x, x, y, y) and (z, z, m, m) per particle. Split form: `hi` = (x, y, z, m)
-// rounded and `lo` = (x - hi, y - hi, z - hi, 0), padded float4 each.
+// `padded` particles. FP32 form (lo == nullptr): padded float4 in `hi`, two per
+// pair of particles, (x0, x1, y0, y1) and (z0, z1, m0, m1). Split form: 2 *
+// padded float4 in each, (x, x, y, y) and (z, z, m, m) per particle in `hi`,
+// rounded, and (x', x', y', y') and (z', z', 0, 0) with x' = x - hi in `lo`.
 cudaError_t pack_sources(const double *x, const double *y, const double *z, const double *m,
                          uint32_t n, uint32_t padded, float4 *hi, float4 *lo,
                          cudaStream_t stream);
 
+// How the parts of a target tile are added: through a cluster's shared memory,
+// or through memory: `sums` of direct_partial_doubles(n, config) and `arrived`
+// of direct_arrival_words(n, config) words, zero before the first launch (each
+// launch leaves them zero). Launches that share them must not overlap.
+struct DirectParts {
+    double *sums = nullptr;
+    unsigned *arrived = nullptr;
+};
+bool direct_uses_cluster(uint32_t n, const DirectConfig &config);
+size_t direct_partial_doubles(uint32_t n, const DirectConfig &config);
+size_t direct_arrival_words(uint32_t n, const DirectConfig &config);
+
 // Plain FP32 direct sum. `sources` is the packed float4 array.
 cudaError_t launch_direct_f32(const float4 *sources, uint32_t n, uint32_t padded, float eps2,
                               double *ax, double *ay, double *az, const DirectConfig &config,
-                              unsigned *status, cudaStream_t stream);
+                              const DirectParts &parts, unsigned *status, cudaStream_t stream);
 
 // Whole integration steps of a small FP32-direct system in one cooperative
 // launch (fused.cu): `steps` steps of `cycle` substeps with timesteps h[0..cycle)
@@ -61,8 +74,8 @@ cudaError_t launch_fused_steps(double *const *state, const double *m, uint32_t n
 // Precision form: hi/lo split positions, Kahan FP32 partials, FP64 tiles.
 cudaError_t launch_direct_split(const float4 *hi, const float4 *lo, uint32_t n, uint32_t padded,
                                 float eps2, double *ax, double *ay, double *az,
-                                const DirectConfig &config, unsigned *status,
-                                cudaStream_t stream);
+                                const DirectConfig &config, const DirectParts &parts,
+                                unsigned *status, cudaStream_t stream);
 
 // FP64 direct sum in the reference scalar kernel's order (bit-identical).
 cudaError_t launch_direct_f64(const double *x, const double *y, const double *z, const double *m,

@@ -125,6 +125,21 @@ DirectConfig Solver::direct_config(uint32_t n) {
     return c;
 }
 
+DirectParts Solver::reserve_parts(uint32_t n, const DirectConfig &config, cudaStream_t stream) {
+    if (direct_uses_cluster(n, config)) {
+        return {};
+    }
+    if (part_sums_.reserve(direct_partial_doubles(n, config))) {
+        ++generation_;
+    }
+    if (part_arrived_.reserve(direct_arrival_words(n, config))) {
+        check(cudaMemsetAsync(part_arrived_.data(), 0, part_arrived_.bytes(), stream),
+              "clearing the arrival words");
+        ++generation_;
+    }
+    return {part_sums_.data(), part_arrived_.data()};
+}
+
 void Solver::evaluate_direct(uint32_t n, const double *x, const double *y, const double *z,
                              const double *m, double *ax, double *ay, double *az,
                              cudaStream_t stream, cudaEvent_t ordered, cudaEvent_t built,
@@ -139,12 +154,13 @@ void Solver::evaluate_direct(uint32_t n, const double *x, const double *y, const
     const bool split = params_.precision == OB_PRECISION_SPLIT;
     const DirectConfig config = direct_config(n);
     const uint32_t padded = direct_padded_count(n, config);
-    if (hi_.reserve(2ull * padded)) {
+    if (hi_.reserve((split ? 2ull : 1ull) * padded)) {
         ++generation_;
     }
     if (split && lo_.reserve(2ull * padded)) {
         ++generation_;
     }
+    const DirectParts parts = reserve_parts(n, config, stream);
     check(pack_sources(x, y, z, m, n, padded, hi_.data(), split ? lo_.data() : nullptr, stream),
           "packing sources");
     record(ordered, stream, external);
@@ -152,11 +168,11 @@ void Solver::evaluate_direct(uint32_t n, const double *x, const double *y, const
     const auto eps2 = static_cast<float>(eps2d);
     if (split) {
         check(launch_direct_split(hi_.data(), lo_.data(), n, padded, eps2, ax, ay, az, config,
-                                  status_.data(), stream),
+                                  parts, status_.data(), stream),
               "split-precision direct kernel");
     } else {
-        check(launch_direct_f32(hi_.data(), n, padded, eps2, ax, ay, az, config, status_.data(),
-                                stream),
+        check(launch_direct_f32(hi_.data(), n, padded, eps2, ax, ay, az, config, parts,
+                                status_.data(), stream),
               "FP32 direct kernel");
     }
 }
@@ -196,7 +212,8 @@ double Solver::autotune(uint32_t n, DirectConfig &chosen) {
             continue;
         }
         const uint32_t padded = direct_padded_count(n, c);
-        hi_.reserve(2ull * padded);
+        hi_.reserve((split ? 2ull : 1ull) * padded);
+        const DirectParts parts = reserve_parts(n, c, stream_);
         if (split) {
             lo_.reserve(2ull * padded);
         }
@@ -206,9 +223,10 @@ double Solver::autotune(uint32_t n, DirectConfig &chosen) {
               "packing autotune sources");
         auto launch = [&]() {
             return split ? launch_direct_split(hi_.data(), lo_.data(), n, padded, eps2, out,
-                                               out + n, out + 2ull * n, c, status_.data(), stream_)
+                                               out + n, out + 2ull * n, c, parts, status_.data(),
+                                               stream_)
                          : launch_direct_f32(hi_.data(), n, padded, eps2, out, out + n,
-                                             out + 2ull * n, c, status_.data(), stream_);
+                                             out + 2ull * n, c, parts, status_.data(), stream_);
         };
         if (launch() != cudaSuccess) {
             cudaGetLastError();

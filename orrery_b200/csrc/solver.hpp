@@ -90,10 +90,16 @@ private:
                          cudaStream_t stream, cudaEvent_t ordered, cudaEvent_t built,
                          bool external);
 
+    // Where the parts of a split source range leave their sums (kept between
+    // evaluations; empty while a cluster adds them).
+    DirectParts reserve_parts(uint32_t n, const DirectConfig &config, cudaStream_t stream);
+
     ob_solver_params params_;
     int sm_count_ = 148;
     DeviceArray<float4> hi_;
     DeviceArray<float4> lo_;
+    DeviceArray<double> part_sums_;
+    DeviceArray<unsigned> part_arrived_;
     DeviceArray<double> staging_;
     DeviceArray<unsigned> status_;
     ob_counts counts_{};
