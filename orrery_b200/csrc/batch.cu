@@ -464,8 +464,10 @@ std::vector<BatchItem> Batch::make_items(const BatchConfig &config,
     for (const uint32_t s : ids) {
         const Member &m = members_[s];
         const uint32_t tiles = ceil_div(m.count, kDirectTile);
-        const uint32_t chunk =
-            config.chunk_tiles == 0 ? tiles : std::min(config.chunk_tiles, tiles);
+        const uint32_t wanted = config.chunk_tiles != kChunkBySize ? config.chunk_tiles
+                                : tiles <= 8u                      ? 2u
+                                                                   : 8u;
+        const uint32_t chunk = wanted == 0 ? tiles : std::min(wanted, tiles);
         const uint32_t chunks = ceil_div(tiles, chunk);
         for (uint32_t t = 0; t < m.count; t += bt) {
             const uint32_t n_targets = std::min(bt, m.count - t);
