@@ -163,12 +163,8 @@ __device__ __forceinline__ uint32_t to_grid(double coordinate, double origin, do
     return __double2uint_rz(cell);
 }
 
-__global__ void __launch_bounds__(kReduceThreads)
-    encode_kernel(const double *__restrict__ x, const double *__restrict__ y,
-                  const double *__restrict__ z, uint32_t n, const TreeMeta *meta,
-                  unsigned long long *codes, uint32_t *indices, uint32_t *hist) {
-    __shared__ unsigned long long table[128];
-    __shared__ uint32_t local[kRadixPasses * kRadix];
+// The dilation table and zeroed local histograms (then a barrier).
+__device__ __forceinline__ void encode_prepare(unsigned long long *table, uint32_t *local) {
     for (uint32_t k = threadIdx.x; k < 128; k += blockDim.x) {
         unsigned long long d = 0;
         for (int b = 0; b < 7; ++b) {
@@ -179,11 +175,20 @@ __global__ void __launch_bounds__(kReduceThreads)
     for (uint32_t k = threadIdx.x; k < kRadixPasses * kRadix; k += blockDim.x) {
         local[k] = 0;
     }
-    __syncthreads();
-    const double size = meta->size;
+}
+
+// This CTA's share of the codes, and its digit counts added to `hist`.
+__device__ __forceinline__ void encode_particles(const double *__restrict__ x,
+                                                 const double *__restrict__ y,
+                                                 const double *__restrict__ z, uint32_t n,
+                                                 const TreeMeta &meta,
+                                                 const unsigned long long *table, uint32_t *local,
+                                                 unsigned long long *codes, uint32_t *indices,
+                                                 uint32_t *hist) {
+    const double size = meta.size;
     const bool degenerate = !(size > 0.0);
     const double scale = degenerate ? 0.0 : __ddiv_rn(2097152.0, size);
-    const double ox = meta->origin[0], oy = meta->origin[1], oz = meta->origin[2];
+    const double ox = meta.origin[0], oy = meta.origin[1], oz = meta.origin[2];
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         unsigned long long code = 0;
         if (!degenerate) {
@@ -204,6 +209,17 @@ __global__ void __launch_bounds__(kReduceThreads)
             atomicAdd(&hist[k], local[k]);
         }
     }
+}
+
+__global__ void __launch_bounds__(kReduceThreads)
+    encode_kernel(const double *__restrict__ x, const double *__restrict__ y,
+                  const double *__restrict__ z, uint32_t n, const TreeMeta *meta,
+                  unsigned long long *codes, uint32_t *indices, uint32_t *hist) {
+    __shared__ unsigned long long table[128];
+    __shared__ uint32_t local[kRadixPasses * kRadix];
+    encode_prepare(table, local);
+    __syncthreads();
+    encode_particles(x, y, z, n, *meta, table, local, codes, indices, hist);
 }
 
 __global__ void scan_histograms_kernel(uint32_t *hist) {
@@ -236,242 +252,340 @@ __device__ __forceinline__ void store_volatile(uint32_t *p, uint32_t v) {
 
 constexpr uint32_t kWarps = kSortThreads / 32;
 
-// One onesweep pass. CTAs are persistent: each takes tiles by atomic ticket
-// (so every tile's predecessors were taken by CTAs that are running or done,
-// which publish without waiting on later tiles) until the tiles run out.
-__global__ void __launch_bounds__(kSortThreads, 5)
-    onesweep_kernel(const unsigned long long *__restrict__ keys_in,
-                    const uint32_t *__restrict__ vals_in, unsigned long long *keys_out,
-                    uint32_t *vals_out, uint32_t n, uint32_t tiles, uint32_t shift,
-                    const uint32_t *__restrict__ offsets, uint32_t *lookback, uint32_t *ticket,
-                    unsigned *status, uint32_t poll_limit) {
-    extern __shared__ __align__(16) unsigned char smem[];
-    unsigned long long *s_keys = reinterpret_cast<unsigned long long *>(smem);
-    uint32_t *s_vals = reinterpret_cast<uint32_t *>(s_keys + kSortTile);
-    uint32_t *s_warp = s_vals + kSortTile;            // [kWarps][kRadix] counts, then prefixes
-    uint32_t *s_start = s_warp + kWarps * kRadix;     // tile-local digit start
-    uint32_t *s_base = s_start + kRadix;              // global output base per digit
-    uint32_t *s_tile = s_base + kRadix;
+// Shared memory of a tile's ranking and scatter.
+struct SortSpace {
+    unsigned long long keys[kSortTile];
+    uint32_t vals[kSortTile];
+    uint32_t warp[kWarps * kRadix]; // counts per warp and digit, then prefixes
+    uint32_t start[kRadix];         // tile-local digit start
+    uint32_t base[kRadix];          // global output base per digit
+    uint32_t sums[kWarps];          // digit counts of each warp's 32 digits
+    uint32_t tile;
+};
 
+// One tile of a pass: ranks its keys stably by digit, publishes its counts,
+// resolves its output bases by looking back over earlier tiles (bounded polls)
+// and scatters. `offset`: where digit threadIdx.x starts in the output.
+// space.warp is zeroed by the caller (and a barrier passed); the caller passes
+// a barrier before it reuses the space. False, in every thread, when a wait ran
+// out.
+__device__ __forceinline__ bool sort_one_tile(SortSpace &space, uint32_t tile,
+                                              const unsigned long long *keys_in,
+                                              const uint32_t *vals_in,
+                                              unsigned long long *keys_out, uint32_t *vals_out,
+                                              uint32_t n, uint32_t shift, uint32_t offset,
+                                              uint32_t *lookback, unsigned *status,
+                                              uint32_t poll_limit) {
+    static_assert(kSortThreads == kRadix, "thread t owns digit t");
+    unsigned long long *s_keys = space.keys;
+    uint32_t *s_vals = space.vals, *s_warp = space.warp, *s_start = space.start;
+    uint32_t *s_base = space.base, *s_sums = space.sums;
     const uint32_t tid = threadIdx.x;
     const uint32_t lane = tid & 31u, warp = tid >> 5;
     const uint32_t lt_mask = (1u << lane) - 1u;
     uint32_t *hist = s_warp + warp * kRadix;
+    const uint32_t base = tile * kSortTile;
+
+    // Warp-striped load: the tile order of (warp, item, lane) is this order.
+    // All of a thread's loads are issued before the ranking's barriers.
+    unsigned long long key[kSortItems];
+    uint32_t val[kSortItems], digit[kSortItems], rank[kSortItems];
+#pragma unroll
+    for (int it = 0; it < kSortItems; ++it) {
+        const uint32_t i = base + warp * (kSortItems * 32) + it * 32 + lane;
+        const bool valid = i < n;
+        key[it] = valid ? __ldcg(keys_in + i) : 0ull;
+        val[it] = valid ? __ldcg(vals_in + i) : 0u;
+    }
+#pragma unroll
+    for (int it = 0; it < kSortItems; ++it) {
+        const bool valid = base + warp * (kSortItems * 32) + it * 32 + lane < n;
+        digit[it] = valid ? static_cast<uint32_t>((key[it] >> shift) & (kRadix - 1)) : kRadix;
+        // Stable warp-local rank: earlier items first, then lower lanes.
+        const uint32_t peers = __match_any_sync(0xffffffffu, digit[it]);
+        const uint32_t before = __popc(peers & lt_mask);
+        const uint32_t running = valid ? hist[digit[it]] : 0u;
+        __syncwarp();
+        if (valid && before == 0) {
+            hist[digit[it]] = running + __popc(peers);
+        }
+        __syncwarp();
+        rank[it] = running + before;
+    }
+    __syncthreads();
+
+    // Thread t owns digit t: tile count, warp prefixes, publish, look back.
+    const uint32_t d = tid;
+    uint32_t count = 0;
+    for (uint32_t w = 0; w < kWarps; ++w) {
+        const uint32_t c = s_warp[w * kRadix + d];
+        s_warp[w * kRadix + d] = count;
+        count += c;
+    }
+    uint32_t *mine = lookback + static_cast<size_t>(tile) * kRadix + d;
+    if (tile == 0) {
+        store_volatile(mine, kFlagPrefix | count);
+    } else {
+        store_volatile(mine, kFlagAggregate | count);
+    }
+    uint32_t exclusive = 0;
+    bool ok = true;
+    if (tile > 0) {
+        int64_t j = static_cast<int64_t>(tile) - 1;
+        uint32_t polls = 0;
+        while (j >= 0) {
+            const uint32_t s = load_volatile(lookback + static_cast<size_t>(j) * kRadix + d);
+            const uint32_t flag = s & ~kCountMask;
+            if (flag == 0u) {
+                if (++polls > poll_limit) {
+                    atomicOr(status, kStatusTimeout);
+                    ok = false;
+                    break;
+                }
+                continue;
+            }
+            exclusive += s & kCountMask;
+            if (flag == kFlagPrefix) {
+                break;
+            }
+            --j;
+        }
+        __threadfence();
+        store_volatile(mine, kFlagPrefix | ((exclusive + count) & kCountMask));
+    }
+    s_base[d] = offset + exclusive;
+
+    // Exclusive scan of the tile's digit counts gives each digit's run start:
+    // within each warp's 32 digits, then over the warps.
+    uint32_t inclusive = count;
+#pragma unroll
+    for (uint32_t off = 1; off < 32; off <<= 1) {
+        const uint32_t v = __shfl_up_sync(0xffffffffu, inclusive, off);
+        inclusive += lane >= off ? v : 0u;
+    }
+    if (lane == 31) {
+        s_sums[warp] = inclusive;
+    }
+    __syncthreads();
+    uint32_t earlier = 0;
+#pragma unroll
+    for (uint32_t w = 0; w < kWarps; ++w) {
+        earlier += w < warp ? s_sums[w] : 0u;
+    }
+    s_start[d] = earlier + inclusive - count;
+    if (!__syncthreads_and(ok ? 1 : 0)) {
+        return false; // a timed-out tile stays unscattered
+    }
+
+    // Place keys in shared memory in digit order, then write contiguous runs.
+#pragma unroll
+    for (int it = 0; it < kSortItems; ++it) {
+        if (digit[it] < kRadix) {
+            const uint32_t pos =
+                s_start[digit[it]] + s_warp[warp * kRadix + digit[it]] + rank[it];
+            s_keys[pos] = key[it];
+            s_vals[pos] = val[it];
+        }
+    }
+    __syncthreads();
+    const uint32_t valid_in_tile = n > base ? min(kSortTile, n - base) : 0u;
+    for (uint32_t k = tid; k < valid_in_tile; k += kSortThreads) {
+        const unsigned long long kk = s_keys[k];
+        const uint32_t dd = static_cast<uint32_t>((kk >> shift) & (kRadix - 1));
+        const uint32_t dst = s_base[dd] + (k - s_start[dd]);
+        keys_out[dst] = kk;
+        vals_out[dst] = s_vals[k];
+    }
+    return true;
+}
+
+// One onesweep pass. CTAs are persistent: each takes tiles by atomic ticket
+// (so every tile's predecessors were taken by CTAs that are running or done,
+// which publish without waiting on later tiles) until the tiles run out.
+__global__ void __launch_bounds__(kSortThreads, 5)
+    onesweep_kernel(const unsigned long long *keys_in, const uint32_t *vals_in,
+                    unsigned long long *keys_out, uint32_t *vals_out, uint32_t n, uint32_t tiles,
+                    uint32_t shift, const uint32_t *__restrict__ offsets, uint32_t *lookback,
+                    uint32_t *ticket, unsigned *status, uint32_t poll_limit) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    SortSpace &space = *reinterpret_cast<SortSpace *>(smem);
+    const uint32_t tid = threadIdx.x;
     while (true) {
         if (tid == 0) {
-            *s_tile = atomicAdd(ticket, 1u);
+            space.tile = atomicAdd(ticket, 1u);
         }
         for (uint32_t k = tid; k < kWarps * kRadix; k += kSortThreads) {
-            s_warp[k] = 0;
+            space.warp[k] = 0;
         }
         __syncthreads();
-        const uint32_t tile = *s_tile;
+        const uint32_t tile = space.tile;
         if (tile >= tiles) {
             return; // uniform: every thread read the same ticket
         }
-        const uint32_t base = tile * kSortTile;
-
-        // Warp-striped load: the tile order of (warp, item, lane) is this order.
-        unsigned long long key[kSortItems];
-        uint32_t val[kSortItems], digit[kSortItems], rank[kSortItems];
-#pragma unroll
-        for (int it = 0; it < kSortItems; ++it) {
-            const uint32_t i = base + warp * (kSortItems * 32) + it * 32 + lane;
-            const bool valid = i < n;
-            key[it] = valid ? keys_in[i] : 0ull;
-            val[it] = valid ? vals_in[i] : 0u;
-            digit[it] = valid ? static_cast<uint32_t>((key[it] >> shift) & (kRadix - 1)) : kRadix;
-            // Stable warp-local rank: earlier items first, then lower lanes.
-            const uint32_t peers = __match_any_sync(0xffffffffu, digit[it]);
-            const uint32_t before = __popc(peers & lt_mask);
-            const uint32_t running = valid ? hist[digit[it]] : 0u;
-            __syncwarp();
-            if (valid && before == 0) {
-                hist[digit[it]] = running + __popc(peers);
-            }
-            __syncwarp();
-            rank[it] = running + before;
-        }
-        __syncthreads();
-
-        // Thread t owns digit t: tile count, warp prefixes, publish, look back.
-        const uint32_t d = tid;
-        uint32_t count = 0;
-        for (uint32_t w = 0; w < kWarps; ++w) {
-            const uint32_t c = s_warp[w * kRadix + d];
-            s_warp[w * kRadix + d] = count;
-            count += c;
-        }
-        uint32_t *mine = lookback + static_cast<size_t>(tile) * kRadix + d;
-        if (tile == 0) {
-            store_volatile(mine, kFlagPrefix | count);
-        } else {
-            store_volatile(mine, kFlagAggregate | count);
-        }
-        uint32_t exclusive = 0;
-        bool ok = true;
-        if (tile > 0) {
-            int64_t j = static_cast<int64_t>(tile) - 1;
-            uint32_t polls = 0;
-            while (j >= 0) {
-                const uint32_t s = load_volatile(lookback + static_cast<size_t>(j) * kRadix + d);
-                const uint32_t flag = s & ~kCountMask;
-                if (flag == 0u) {
-                    if (++polls > poll_limit) {
-                        atomicOr(status, kStatusTimeout);
-                        ok = false;
-                        break;
-                    }
-                    continue;
-                }
-                exclusive += s & kCountMask;
-                if (flag == kFlagPrefix) {
-                    break;
-                }
-                --j;
-            }
-            __threadfence();
-            store_volatile(mine, kFlagPrefix | ((exclusive + count) & kCountMask));
-        }
-        s_base[d] = offsets[d] + exclusive;
-
-        // Exclusive scan of the tile's digit counts gives each digit's run start.
-        s_start[d] = count;
-        __syncthreads();
-        for (uint32_t off = 1; off < kRadix; off <<= 1) {
-            const uint32_t v = d >= off ? s_start[d - off] : 0u;
-            __syncthreads();
-            s_start[d] += v;
-            __syncthreads();
-        }
-        s_start[d] -= count;
-        __syncthreads();
-        if (!__syncthreads_and(ok ? 1 : 0)) {
-            return; // a timed-out tile stays unscattered; the CTA takes no more tiles
-        }
-
-        // Place keys in shared memory in digit order, then write contiguous runs.
-#pragma unroll
-        for (int it = 0; it < kSortItems; ++it) {
-            if (digit[it] < kRadix) {
-                const uint32_t pos =
-                    s_start[digit[it]] + s_warp[warp * kRadix + digit[it]] + rank[it];
-                s_keys[pos] = key[it];
-                s_vals[pos] = val[it];
-            }
-        }
-        __syncthreads();
-        const uint32_t valid_in_tile = n > base ? min(kSortTile, n - base) : 0u;
-        for (uint32_t k = tid; k < valid_in_tile; k += kSortThreads) {
-            const unsigned long long kk = s_keys[k];
-            const uint32_t dd = static_cast<uint32_t>((kk >> shift) & (kRadix - 1));
-            const uint32_t dst = s_base[dd] + (k - s_start[dd]);
-            keys_out[dst] = kk;
-            vals_out[dst] = s_vals[k];
+        if (!sort_one_tile(space, tile, keys_in, vals_in, keys_out, vals_out, n, shift,
+                           offsets[tid], lookback, status, poll_limit)) {
+            return; // the CTA takes no more tiles
         }
         __syncthreads(); // the next tile reuses the shared arrays
     }
 }
 
-__global__ void gather_kernel(const double *__restrict__ x, const double *__restrict__ y,
-                              const double *__restrict__ z, const double *__restrict__ m,
-                              const uint32_t *__restrict__ perm, uint32_t n, double *sorted) {
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const uint32_t j = perm[i];
-        sorted[i] = x[j];
-        sorted[static_cast<size_t>(n) + i] = y[j];
-        sorted[2ull * n + i] = z[j];
-        sorted[3ull * n + i] = m[j];
-    }
-}
+// The whole ordering in one cooperative launch: cube, codes and digit
+// histograms, eight sort passes and the gather, with a grid barrier between
+// phases. An evaluation made of one launch per phase spent 90 us of host time
+// on the ordering's launches and clears whatever the size (a 10,000-particle
+// evaluation 309 us, of which the walk 117).
+struct OrderArgs {
+    const double *x, *y, *z, *m;
+    uint32_t n, tiles;
+    unsigned long long *keys[2];
+    uint32_t *perm[2];
+    uint32_t *hist;
+    uint32_t *lookback; // of all passes
+    double *partials;   // 6 per CTA
+    double *sorted;
+    uint32_t *zeroed;   // words of the construction to zero on the way
+    size_t zeroed_words;
+    TreeMeta *meta;
+    unsigned *barrier;
+    unsigned *status;
+};
 
-// Three-phase exclusive scan: block sums, a scan of the sums, block scans.
-constexpr uint32_t kScanThreads = 256;
-constexpr uint32_t kScanItems = 16;
-constexpr uint32_t kScanTile = kScanThreads * kScanItems;
+struct OrderSpace {
+    union {
+        SortSpace sort;
+        struct {
+            unsigned long long table[128];
+            uint32_t local[kRadixPasses * kRadix];
+        } encode;
+    };
+};
 
-__device__ uint32_t block_exclusive_scan(uint32_t v, uint32_t *s, uint32_t &total) {
-    const uint32_t t = threadIdx.x;
-    s[t] = v;
-    __syncthreads();
-    for (uint32_t off = 1; off < blockDim.x; off <<= 1) {
-        const uint32_t u = t >= off ? s[t - off] : 0u;
-        __syncthreads();
-        s[t] += u;
-        __syncthreads();
-    }
-    total = s[blockDim.x - 1];
-    const uint32_t r = s[t] - v;
-    __syncthreads();
-    return r;
-}
+__global__ void __launch_bounds__(kSortThreads, 4) order_kernel(const OrderArgs a) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    OrderSpace &space = *reinterpret_cast<OrderSpace *>(smem);
+    __shared__ TreeMeta cube;
+    __shared__ double ext[6];
+    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+    const uint32_t first = blockIdx.x * kSortThreads + tid, stride = gridDim.x * kSortThreads;
+    unsigned barriers = 0;
 
-__global__ void __launch_bounds__(kScanThreads)
-    scan_reduce_kernel(const uint32_t *__restrict__ in, uint32_t n, uint32_t *sums) {
-    __shared__ uint32_t s[kScanThreads];
-    const uint32_t base = blockIdx.x * kScanTile;
-    uint32_t local = 0;
-    for (uint32_t k = 0; k < kScanItems; ++k) {
-        const uint32_t i = base + k * kScanThreads + threadIdx.x;
-        local += i < n ? in[i] : 0u;
+    // Nothing reads these words before the first barrier.
+    for (size_t k = first; k < static_cast<size_t>(kRadixPasses) * kRadix; k += stride) {
+        a.hist[k] = 0u;
     }
-    uint32_t total;
-    block_exclusive_scan(local, s, total);
-    if (threadIdx.x == 0) {
-        sums[blockIdx.x] = total;
+    for (size_t k = first; k < static_cast<size_t>(kRadixPasses) * a.tiles * kRadix; k += stride) {
+        a.lookback[k] = 0u;
     }
-}
+    for (size_t k = first; k < a.zeroed_words; k += stride) {
+        a.zeroed[k] = 0u;
+    }
 
-__global__ void __launch_bounds__(1024) scan_sums_kernel(uint32_t *sums, uint32_t blocks) {
-    __shared__ uint32_t s[1024];
-    uint32_t carry = 0;
-    for (uint32_t start = 0; start < blocks; start += 1024) {
-        const uint32_t i = start + threadIdx.x;
-        const uint32_t v = i < blocks ? sums[i] : 0u;
-        uint32_t total;
-        const uint32_t r = block_exclusive_scan(v, s, total);
-        if (i < blocks) {
-            sums[i] = carry + r;
-        }
-        carry += total;
+    // The extremes: each CTA's, then (after the barrier) all CTAs' folded by
+    // every CTA alike (min and max are exact in any order).
+    double v[6] = {INFINITY, INFINITY, INFINITY, -INFINITY, -INFINITY, -INFINITY};
+    for (uint32_t i = first; i < a.n; i += stride) {
+        min_max(a.x[i], v[0], v[3]);
+        min_max(a.y[i], v[1], v[4]);
+        min_max(a.z[i], v[2], v[5]);
     }
-    if (threadIdx.x == 0) {
-        sums[blocks] = carry;
+    double mine = 0.0;
+    block_min_max(v, mine);
+    if (tid < 6) {
+        a.partials[blockIdx.x * 6 + tid] = mine;
     }
-}
-
-__global__ void __launch_bounds__(kScanThreads)
-    scan_apply_kernel(const uint32_t *__restrict__ in, uint32_t *out, uint32_t n,
-                      const uint32_t *sums, uint32_t blocks) {
-    __shared__ uint32_t s[kScanThreads];
-    const uint32_t base = blockIdx.x * kScanTile + threadIdx.x * kScanItems;
-    uint32_t v[kScanItems];
-    uint32_t local = 0;
+    if (!grid_barrier(a.barrier, ++barriers, a.status)) {
+        return;
+    }
 #pragma unroll
-    for (uint32_t k = 0; k < kScanItems; ++k) {
-        const uint32_t i = base + k;
-        v[k] = i < n ? in[i] : 0u;
-        local += v[k];
+    for (int k = 0; k < 6; ++k) {
+        v[k] = k < 3 ? INFINITY : -INFINITY;
     }
-    uint32_t total;
-    uint32_t running = sums[blockIdx.x] + block_exclusive_scan(local, s, total);
+    for (uint32_t b = tid; b < gridDim.x; b += kSortThreads) {
 #pragma unroll
-    for (uint32_t k = 0; k < kScanItems; ++k) {
-        const uint32_t i = base + k;
-        if (i < n) {
-            out[i] = running;
+        for (int k = 0; k < 6; ++k) {
+            // Empty CTAs hold (+inf, -inf): lows only lower, highs only raise.
+            const double p = __ldcg(a.partials + b * 6 + k);
+            v[k] = k < 3 ? (p < v[k] ? p : v[k]) : (v[k] < p ? p : v[k]);
         }
-        running += v[k];
     }
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        out[n] = sums[blocks];
+    double folded = 0.0;
+    block_min_max(v, folded);
+    if (tid < 6) {
+        ext[tid] = folded;
+    }
+    __syncthreads();
+    if (tid == 0) {
+        cube = TreeMeta{};
+        write_cube(ext, a.n, &cube);
+        if (blockIdx.x == 0) {
+            *a.meta = cube; // the other scalars start at zero
+        }
+    }
+    encode_prepare(space.encode.table, space.encode.local);
+    __syncthreads();
+    encode_particles(a.x, a.y, a.z, a.n, cube, space.encode.table, space.encode.local, a.keys[0],
+                     a.perm[0], a.hist);
+    if (!grid_barrier(a.barrier, ++barriers, a.status)) {
+        return;
+    }
+
+    for (int pass = 0; pass < kRadixPasses; ++pass) {
+        const bool odd = (pass & 1) != 0;
+        const unsigned long long *keys_in = odd ? a.keys[1] : a.keys[0];
+        unsigned long long *keys_out = odd ? a.keys[0] : a.keys[1];
+        const uint32_t *perm_in = odd ? a.perm[1] : a.perm[0];
+        uint32_t *perm_out = odd ? a.perm[0] : a.perm[1];
+        if (blockIdx.x < a.tiles) {
+            // Where digit `tid` starts in the output: the exclusive scan of the
+            // pass's histogram.
+            const uint32_t count = __ldcg(a.hist + pass * kRadix + tid);
+            uint32_t inclusive = count;
+#pragma unroll
+            for (uint32_t off = 1; off < 32; off <<= 1) {
+                const uint32_t u = __shfl_up_sync(0xffffffffu, inclusive, off);
+                inclusive += lane >= off ? u : 0u;
+            }
+            if (lane == 31) {
+                space.sort.sums[warp] = inclusive;
+            }
+            __syncthreads();
+            uint32_t offset = inclusive - count;
+#pragma unroll
+            for (uint32_t w = 0; w < kWarps; ++w) {
+                offset += w < warp ? space.sort.sums[w] : 0u;
+            }
+            // Ascending tiles per CTA: the lowest unfinished tile waits for none.
+            for (uint32_t tile = blockIdx.x; tile < a.tiles; tile += gridDim.x) {
+                __syncthreads(); // the previous tile's (or the sums') last readers
+                for (uint32_t k = tid; k < kWarps * kRadix; k += kSortThreads) {
+                    space.sort.warp[k] = 0;
+                }
+                __syncthreads();
+                if (!sort_one_tile(space.sort, tile, keys_in, perm_in, keys_out, perm_out, a.n,
+                                   static_cast<uint32_t>(kRadixBits * pass), offset,
+                                   a.lookback + static_cast<size_t>(pass) * a.tiles * kRadix,
+                                   a.status, kLookbackPollLimit)) {
+                    return; // the status word tells; the other CTAs' waits run out too
+                }
+            }
+        }
+        if (!grid_barrier(a.barrier, ++barriers, a.status)) {
+            return;
+        }
+    }
+
+    // Eight passes end in buffer 0.
+    for (uint32_t i = first; i < a.n; i += stride) {
+        const uint32_t j = __ldcg(a.perm[0] + i);
+        a.sorted[i] = a.x[j];
+        a.sorted[static_cast<size_t>(a.n) + i] = a.y[j];
+        a.sorted[2ull * a.n + i] = a.z[j];
+        a.sorted[3ull * a.n + i] = a.m[j];
     }
 }
 
-size_t onesweep_smem() {
-    return kSortTile * (sizeof(unsigned long long) + sizeof(uint32_t)) +
-           (kWarps * kRadix + 2 * kRadix + 4) * sizeof(uint32_t);
-}
+size_t onesweep_smem() { return sizeof(SortSpace); }
 
 } // namespace
 
@@ -535,22 +649,52 @@ cudaError_t launch_onesweep(const unsigned long long *keys_in, const uint32_t *v
     return cudaGetLastError();
 }
 
-cudaError_t launch_gather(const double *x, const double *y, const double *z, const double *m,
-                          const uint32_t *perm, uint32_t n, double *sorted, cudaStream_t stream) {
-    const uint32_t blocks = max(1u, min(ceil_div(n, 256), 148u * 16u));
-    gather_kernel<<<blocks, 256, 0, stream>>>(x, y, z, m, perm, n, sorted);
-    return cudaGetLastError();
+cudaError_t cooperative_grid(const void *kernel, int threads, size_t smem,
+                             std::atomic<uint64_t> &configured, std::atomic<int> &resident,
+                             uint32_t wanted, uint32_t &grid) {
+    cudaError_t err = set_smem_limit_once(kernel, static_cast<int>(smem), configured);
+    if (err == cudaSuccess && resident.load(std::memory_order_relaxed) == 0) {
+        int per_sm = 0, sms = 0, device = 0;
+        err = cudaGetDevice(&device);
+        if (err == cudaSuccess) {
+            err = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+        }
+        if (err == cudaSuccess) {
+            err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem);
+        }
+        if (err == cudaSuccess) {
+            resident.store(std::max(1, per_sm) * std::max(1, sms), std::memory_order_relaxed);
+        }
+    }
+    grid = std::max(1u, std::min(wanted, static_cast<uint32_t>(resident.load())));
+    return err;
 }
 
-size_t scan_partials_needed(uint32_t n) { return ceil_div(n == 0 ? 1 : n, kScanTile) + 1ull; }
+size_t order_partials_needed() { return 6ull * kMaxCooperativeBlocks; }
 
-cudaError_t launch_exclusive_scan(const uint32_t *in, uint32_t *out, uint32_t n,
-                                  uint32_t *scratch, cudaStream_t stream) {
-    const uint32_t blocks = ceil_div(n == 0 ? 1 : n, kScanTile);
-    scan_reduce_kernel<<<blocks, kScanThreads, 0, stream>>>(in, n, scratch);
-    scan_sums_kernel<<<1, 1024, 0, stream>>>(scratch, blocks);
-    scan_apply_kernel<<<blocks, kScanThreads, 0, stream>>>(in, out, n, scratch, blocks);
-    return cudaGetLastError();
+cudaError_t launch_order(const double *x, const double *y, const double *z, const double *m,
+                         uint32_t n, unsigned long long *const *keys, uint32_t *const *perm,
+                         uint32_t *hist, uint32_t *lookback, double *partials, double *sorted,
+                         uint32_t *zeroed, size_t zeroed_words, TreeMeta *meta,
+                         unsigned *barrier, unsigned *status, cudaStream_t stream) {
+    static std::atomic<uint64_t> configured{0};
+    static std::atomic<int> resident{0};
+    const void *kernel = reinterpret_cast<const void *>(order_kernel);
+    const uint32_t tiles = sort_tiles(n);
+    uint32_t grid = 0;
+    const cudaError_t err =
+        cooperative_grid(kernel, kSortThreads, sizeof(OrderSpace), configured, resident,
+                         std::min(std::max(tiles, ceil_div(n, 1024u)), kMaxCooperativeBlocks),
+                         grid);
+    if (err != cudaSuccess) {
+        return err;
+    }
+    OrderArgs a{x,        y,      z,      m,            n,    tiles,   {keys[0], keys[1]},
+                {perm[0], perm[1]}, hist,   lookback,     partials, sorted, zeroed,
+                zeroed_words,       meta,   barrier,      status};
+    void *args[] = {&a};
+    return cudaLaunchCooperativeKernel(kernel, dim3(grid), dim3(kSortThreads), args,
+                                       sizeof(OrderSpace), stream);
 }
 
 } // namespace ob

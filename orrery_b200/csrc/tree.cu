@@ -24,6 +24,7 @@
 // octree.cpp:75-185, 374-387), so masses, centres of mass, quadrupoles and
 // acceptance radii are bit-identical to the reference's.
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <vector>
 
@@ -36,6 +37,9 @@ namespace {
 
 constexpr uint32_t kLevels = 21;
 constexpr uint32_t kThreads = 256;
+// Words of the scratch before the histograms: the ordering's and the layout's
+// barrier counts.
+constexpr size_t kBarrierWords = 4;
 
 // Leading octal digits (levels) that codes a and b share; kLevels when equal.
 __device__ __forceinline__ int shared_levels(unsigned long long a, unsigned long long b) {
@@ -181,31 +185,98 @@ __device__ void node_run(const unsigned long long *codes, uint32_t n, uint32_t c
     }
 }
 
-__global__ void __launch_bounds__(kThreads)
-    layout_count_kernel(const unsigned long long *__restrict__ codes, uint32_t n, uint32_t cap,
-                        uint32_t *counts) {
-    for (uint32_t b = blockIdx.x * blockDim.x + threadIdx.x; b < n; b += gridDim.x * blockDim.x) {
-        int c;
-        uint32_t lo, hi;
-        node_run(codes, n, cap, b, c, lo, hi);
-        counts[b] = lo <= hi ? hi - lo + 1 : 0u;
+// Node counts, their prefix sums and the node records in one cooperative
+// launch, with two grid barriers. Each CTA owns a contiguous share of the
+// particles; the prefix of a share is the sum of the totals before it.
+__global__ void __launch_bounds__(kThreads, 4)
+    layout_kernel(const unsigned long long *__restrict__ codes, uint32_t n, uint32_t cap,
+                  uint32_t *offsets, uint32_t *totals, uint32_t capacity, DeviceNode *nodes,
+                  uint32_t *child_mask, uint32_t *child_slots, TreeMeta *meta, unsigned *barrier,
+                  unsigned *status) {
+    __shared__ uint32_t sums[kThreads / 32];
+    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+    const uint32_t share = (n + gridDim.x - 1u) / gridDim.x;
+    const uint32_t share_begin = min(static_cast<uint64_t>(blockIdx.x) * share,
+                                     static_cast<uint64_t>(n));
+    const uint32_t share_end = min(static_cast<uint64_t>(share_begin) + share,
+                                   static_cast<uint64_t>(n));
+    // Counts and their exclusive prefix within the share.
+    uint32_t carry = 0;
+    for (uint32_t base = share_begin; base < share_end; base += kThreads) {
+        const uint32_t b = base + tid;
+        uint32_t count = 0;
+        if (b < share_end) {
+            int c;
+            uint32_t lo, hi;
+            node_run(codes, n, cap, b, c, lo, hi);
+            count = lo <= hi ? hi - lo + 1 : 0u;
+        }
+        uint32_t inclusive = count;
+#pragma unroll
+        for (uint32_t off = 1; off < 32; off <<= 1) {
+            const uint32_t v = __shfl_up_sync(0xffffffffu, inclusive, off);
+            inclusive += lane >= off ? v : 0u;
+        }
+        if (lane == 31) {
+            sums[warp] = inclusive;
+        }
+        __syncthreads();
+        uint32_t before = 0, all = 0;
+#pragma unroll
+        for (uint32_t w = 0; w < kThreads / 32; ++w) {
+            before += w < warp ? sums[w] : 0u;
+            all += sums[w];
+        }
+        if (b < share_end) {
+            offsets[b] = carry + before + inclusive - count;
+        }
+        carry += all;
+        __syncthreads();
     }
-}
-
-__global__ void __launch_bounds__(kThreads)
-    layout_write_kernel(const unsigned long long *__restrict__ codes, uint32_t n, uint32_t cap,
-                        const uint32_t *__restrict__ offsets, uint32_t capacity,
-                        DeviceNode *nodes, uint32_t *child_mask, uint32_t *child_slots,
-                        TreeMeta *meta, unsigned *status) {
+    if (tid == 0) {
+        totals[blockIdx.x] = carry;
+    }
+    if (!grid_barrier(barrier, 1u, status)) {
+        return;
+    }
+    // The nodes before this share, and all of them.
+    uint32_t before = 0, total = 0;
+    for (uint32_t q = tid; q < gridDim.x; q += kThreads) {
+        const uint32_t t = __ldcg(totals + q);
+        before += q < blockIdx.x ? t : 0u;
+        total += t;
+    }
+    __shared__ uint32_t folded[2];
+    if (tid < 2) {
+        folded[tid] = 0u;
+    }
+    __syncthreads();
+    before = __reduce_add_sync(0xffffffffu, before);
+    total = __reduce_add_sync(0xffffffffu, total);
+    if (lane == 0) {
+        atomicAdd(&folded[0], before);
+        atomicAdd(&folded[1], total);
+    }
+    __syncthreads();
+    before = folded[0];
+    total = folded[1];
+    for (uint32_t b = share_begin + tid; b < share_end; b += kThreads) {
+        offsets[b] += before; // this thread wrote it
+    }
+    if (blockIdx.x == 0 && tid == 0) {
+        offsets[n] = total;
+    }
+    if (!grid_barrier(barrier, 2u, status)) {
+        return;
+    }
     if (blockIdx.x == 0 && threadIdx.x == 0) {
-        const uint32_t total = offsets[n];
         meta->node_count = total <= capacity ? total : 0u;
         meta->required = total;
         if (total > capacity) {
             atomicOr(status, kStatusOverflow);
         }
     }
-    if (offsets[n] > capacity) {
+    if (total > capacity) {
         return;
     }
     uint32_t leaves = 0, depth = 0;
@@ -216,7 +287,7 @@ __global__ void __launch_bounds__(kThreads)
         if (lo > hi) {
             continue;
         }
-        uint32_t index = offsets[b];
+        uint32_t index = __ldcg(offsets + b);
         uint32_t parent;
         if (b == 0) {
             parent = index; // the root is its own parent
@@ -227,7 +298,7 @@ __global__ void __launch_bounds__(kThreads)
             const uint32_t start = cell_start(codes, b - 1, level);
             const int cs = common_levels(codes, start);
             const uint32_t first_level = start == 0 ? 0u : static_cast<uint32_t>(cs + 1);
-            parent = offsets[start] + (level - first_level);
+            parent = __ldcg(offsets + start) + (level - first_level);
         }
         for (uint32_t level = lo; level <= hi; ++level, ++index) {
             const bool leaf = level == hi;
@@ -238,7 +309,7 @@ __global__ void __launch_bounds__(kThreads)
             node.com_x = node.com_y = node.com_z = 0.0;
             node.r2 = 0.0;
             node.mass = 0.0;
-            node.next = offsets[end];
+            node.next = __ldcg(offsets + end);
             node.count = leaf ? end - b : 0u;
             node.first = b;
             node.level = level;
@@ -538,20 +609,24 @@ uint32_t grid_for(uint32_t n) { return std::max(1u, std::min(ceil_div(n, kThread
 
 } // namespace
 
-cudaError_t launch_layout_count(const unsigned long long *codes, uint32_t n, uint32_t leaf_cap,
-                                uint32_t *counts, cudaStream_t stream) {
-    layout_count_kernel<<<grid_for(n), kThreads, 0, stream>>>(codes, n, leaf_cap, counts);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_layout_write(const unsigned long long *codes, uint32_t n, uint32_t leaf_cap,
-                                const uint32_t *offsets, uint32_t node_capacity,
-                                DeviceNode *nodes, uint32_t *child_mask, uint32_t *child_slots,
-                                TreeMeta *meta, unsigned *status, cudaStream_t stream) {
-    layout_write_kernel<<<grid_for(n), kThreads, 0, stream>>>(codes, n, leaf_cap, offsets,
-                                                             node_capacity, nodes, child_mask,
-                                                             child_slots, meta, status);
-    return cudaGetLastError();
+cudaError_t launch_layout(const unsigned long long *codes, uint32_t n, uint32_t leaf_cap,
+                          uint32_t *offsets, uint32_t *totals, uint32_t node_capacity,
+                          DeviceNode *nodes, uint32_t *child_mask, uint32_t *child_slots,
+                          TreeMeta *meta, unsigned *barrier, unsigned *status,
+                          cudaStream_t stream) {
+    static std::atomic<uint64_t> configured{0};
+    static std::atomic<int> resident{0};
+    const void *kernel = reinterpret_cast<const void *>(layout_kernel);
+    uint32_t grid = 0;
+    const cudaError_t err = cooperative_grid(kernel, kThreads, 0, configured, resident,
+                                             std::min(ceil_div(n, kThreads), kMaxCooperativeBlocks),
+                                             grid);
+    if (err != cudaSuccess) {
+        return err;
+    }
+    void *args[] = {&codes,        &n,     &leaf_cap,   &offsets,     &totals, &node_capacity,
+                    &nodes,        &child_mask, &child_slots, &meta,  &barrier, &status};
+    return cudaLaunchCooperativeKernel(kernel, dim3(grid), dim3(kThreads), args, 0, stream);
 }
 
 cudaError_t launch_moments(const double *sorted, const unsigned long long *codes, uint32_t n,
@@ -602,14 +677,13 @@ void TreePipeline::reserve(uint32_t n) {
             keys_[k].reserve(n);
             perm_[k].reserve(n);
         }
+        scratch_.reserve(kBarrierWords + kRadixPasses * kRadix +
+                         static_cast<size_t>(kRadixPasses) * sort_tiles(n) * kRadix);
         sorted_.reserve(4ull * n);
         leaf_rel_.reserve(n);
-        node_start_.reserve(2ull * n + 1);
-        scan_partials_.reserve(scan_partials_needed(n));
-        reduce_.reserve(cube_partials_needed(n));
-        hist_.reserve(kRadixPasses * kRadix);
-        lookback_.reserve(static_cast<size_t>(kRadixPasses) * sort_tiles(n) * kRadix);
-        tile_counter_.reserve(kRadixPasses);
+        node_start_.reserve(n + 1ull);
+        scan_partials_.reserve(kMaxCooperativeBlocks);
+        reduce_.reserve(order_partials_needed());
         capacity_ = n;
     }
     const uint32_t want = std::max(nodes_for(n), grow_to_);
@@ -640,55 +714,37 @@ void TreePipeline::evaluate(uint32_t n, const double *x, const double *y, const 
     }
     reserve(n);
     last_n_ = n;
-    const uint32_t tiles = sort_tiles(n);
-    // Per-evaluation scalars and scratch.
-    check(cudaMemsetAsync(meta_.data(), 0, sizeof(TreeMeta), stream), "clearing tree scalars");
-    check(cudaMemsetAsync(hist_.data(), 0, hist_.bytes(), stream), "clearing histograms");
-    check(cudaMemsetAsync(lookback_.data(), 0,
-                          sizeof(uint32_t) * kRadixPasses * static_cast<size_t>(tiles) * kRadix,
-                          stream),
-          "clearing look-back words");
-    check(cudaMemsetAsync(tile_counter_.data(), 0, sizeof(uint32_t) * kRadixPasses, stream),
-          "clearing tile tickets");
-    check(cudaMemsetAsync(level_lists_.data() + kMaxChildren * static_cast<size_t>(node_capacity_),
-                          0, sizeof(uint32_t) * 2ull * node_capacity_, stream),
-          "clearing child masks");
-
-    // Ordering: cube, codes + histograms, eight onesweep passes, gather.
-    check(launch_bounding_cube(x, y, z, n, reduce_.data(), meta_.data(), stream), "cube");
-    check(launch_encode(x, y, z, n, meta_.data(), keys_[0].data(), perm_[0].data(), hist_.data(),
-                        stream),
-          "Morton codes");
-    check(launch_scan_histograms(hist_.data(), stream), "digit offsets");
-    for (int pass = 0; pass < kRadixPasses; ++pass) {
-        const int src = pass & 1;
-        check(launch_onesweep(keys_[src].data(), perm_[src].data(), keys_[1 - src].data(),
-                              perm_[1 - src].data(), n, pass, hist_.data(),
-                              lookback_.data() + static_cast<size_t>(pass) * tiles * kRadix,
-                              tile_counter_.data() + pass, status, stream),
-              "radix sort pass");
-    }
-    // Eight passes end in buffer 0.
-    const unsigned long long *codes = keys_[0].data();
-    const uint32_t *perm = perm_[0].data();
-    check(launch_gather(x, y, z, m, perm, n, sorted_.data(), stream), "gather");
-    record(ordered, stream, external);
-
-    // Construction: layout, node offsets, records, moments.
-    const uint32_t cap = static_cast<uint32_t>(std::min<uint64_t>(params_.leaf_capacity,
-                                                                 0xffffffffull));
-    uint32_t *counts = node_start_.data();
-    uint32_t *offsets = node_start_.data() + n;
-    check(launch_layout_count(codes, n, cap, counts, stream), "node counts");
-    check(launch_exclusive_scan(counts, offsets, n, scan_partials_.data(), stream), "node scan");
+    unsigned *barriers = scratch_.data();
+    uint32_t *hist = scratch_.data() + kBarrierWords;
+    uint32_t *lookback = hist + kRadixPasses * kRadix;
     uint32_t *child_slots = level_lists_.data();
     uint32_t *child_mask = child_slots + kMaxChildren * static_cast<size_t>(node_capacity_);
     uint32_t *arrived = child_mask + node_capacity_;
+    check(cudaMemsetAsync(barriers, 0, sizeof(unsigned) * kBarrierWords, stream),
+          "clearing the barriers");
+
+    // Ordering: cube, codes, radix sort, gather; codes and permutation end in
+    // buffer 0.
+    unsigned long long *keys[2] = {keys_[0].data(), keys_[1].data()};
+    uint32_t *perms[2] = {perm_[0].data(), perm_[1].data()};
+    check(launch_order(x, y, z, m, n, keys, perms, hist, lookback, reduce_.data(),
+                       sorted_.data(), child_mask, 2ull * node_capacity_, meta_.data(), barriers,
+                       status, stream),
+          "ordering");
+    const unsigned long long *codes = keys_[0].data();
+    const uint32_t *perm = perm_[0].data();
+    record(ordered, stream, external);
+
+    // Construction: node offsets and records, moments.
+    const uint32_t cap = static_cast<uint32_t>(std::min<uint64_t>(params_.leaf_capacity,
+                                                                 0xffffffffull));
+    uint32_t *offsets = node_start_.data();
     float4 *records = walk_records_.data();
     const WalkNodes walk{records, records + node_capacity_, records + 2ull * node_capacity_,
                          records + 3ull * node_capacity_, walk_index_.data()};
-    check(launch_layout_write(codes, n, cap, offsets, node_capacity_, nodes_.data(), child_mask,
-                              child_slots, meta_.data(), status, stream),
+    check(launch_layout(codes, n, cap, offsets, scan_partials_.data(), node_capacity_,
+                        nodes_.data(), child_mask, child_slots, meta_.data(), barriers + 1,
+                        status, stream),
           "node layout");
     check(launch_moments(sorted_.data(), codes, n, nodes_.data(),
                          params_.quadrupole ? quads_.data() : nullptr, walk, child_mask,

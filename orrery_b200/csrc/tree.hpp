@@ -128,13 +128,12 @@ private:
     int sm_count_ = 148;
     DeviceArray<unsigned long long> keys_[2];    // Morton codes (double-buffered)
     DeviceArray<uint32_t> perm_[2];              // particle index payload
-    DeviceArray<uint32_t> hist_;                 // digit histograms, then offsets
-    DeviceArray<uint32_t> lookback_;             // onesweep tile status words
-    DeviceArray<uint32_t> tile_counter_;         // onesweep tile tickets
+    DeviceArray<uint32_t> scratch_;              // barrier counts, digit histograms, look-back
+                                                 // words
     DeviceArray<double> sorted_;                 // x, y, z, m in Morton order (FP64)
     DeviceArray<float4> leaf_rel_;               // FP32 position - leaf centre of mass, mass
-    DeviceArray<uint32_t> node_start_;           // nodes starting at each particle + scan
-    DeviceArray<uint32_t> scan_partials_;        // block sums of the scan
+    DeviceArray<uint32_t> node_start_;           // nodes that start before each particle
+    DeviceArray<uint32_t> scan_partials_;        // node totals of the layout's CTAs
     DeviceArray<DeviceNode> nodes_;
     DeviceArray<DeviceQuadrupole> quads_;        // FP64 moments (parity, upward pass)
     DeviceArray<float4> walk_records_;           // compact FP32 node records the walk reads

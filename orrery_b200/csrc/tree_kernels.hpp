@@ -2,6 +2,7 @@
 // walk.cu). Raw device pointers; every launcher enqueues on `stream` only.
 #pragma once
 
+#include <atomic>
 #include <cstdint>
 
 #include <cuda_runtime.h>
@@ -59,31 +60,39 @@ cudaError_t launch_onesweep(const unsigned long long *keys_in, const uint32_t *v
                             uint32_t *ticket, unsigned *status, cudaStream_t stream,
                             uint32_t poll_limit = kLookbackPollLimit);
 
-// sorted[k * n + i] = source_k[perm[i]] for x, y, z, m.
-cudaError_t launch_gather(const double *x, const double *y, const double *z, const double *m,
-                          const uint32_t *perm, uint32_t n, double *sorted, cudaStream_t stream);
+// CTAs of a cooperative launch: as many as are resident at once, at most
+// `wanted`. `configured` and `resident` are the caller's per-kernel caches.
+constexpr uint32_t kMaxCooperativeBlocks = 592; // 4 per SM
+cudaError_t cooperative_grid(const void *kernel, int threads, size_t smem,
+                             std::atomic<uint64_t> &configured, std::atomic<int> &resident,
+                             uint32_t wanted, uint32_t &grid);
 
-// Exclusive scan of n uint32 values into out[0..n] (out[n] = total). `scratch`
-// holds scan_partials_needed(n) words.
-size_t scan_partials_needed(uint32_t n);
-cudaError_t launch_exclusive_scan(const uint32_t *in, uint32_t *out, uint32_t n,
-                                  uint32_t *scratch, cudaStream_t stream);
+// The whole ordering in one cooperative launch: the bounding cube into meta,
+// codes (ending in keys[0]) and the permutation (perm[0]), and sorted[k * n + i]
+// = source_k[perm[0][i]] for x, y, z, m; *meta's other scalars and the
+// `zeroed_words` words at `zeroed` are zeroed on the way. `barrier` (one word)
+// is zero at the start; hist, lookback (of all passes) and `partials`
+// (order_partials_needed() doubles) are scratch.
+size_t order_partials_needed();
+cudaError_t launch_order(const double *x, const double *y, const double *z, const double *m,
+                         uint32_t n, unsigned long long *const *keys, uint32_t *const *perm,
+                         uint32_t *hist, uint32_t *lookback, double *partials, double *sorted,
+                         uint32_t *zeroed, size_t zeroed_words, TreeMeta *meta,
+                         unsigned *barrier, unsigned *status, cudaStream_t stream);
 
 // ------------------------------------------------------------------ octree
 
-// Per sorted particle b: the number of octree nodes whose first particle is b.
-cudaError_t launch_layout_count(const unsigned long long *codes, uint32_t n, uint32_t leaf_cap,
-                                uint32_t *counts, cudaStream_t stream);
-
-// Writes the node records (escape, first, count, level, parent, octant), marks
-// each internal node's children by octant in child_mask (zeroed beforehand) and
-// lists them in its kMaxChildren child_slots, one per octant. `offsets` is the
-// exclusive scan of counts.
+// The octree's layout in one cooperative launch: offsets[b] = nodes whose first
+// particle comes before b (n + 1 words), the node records (escape, first, count,
+// level, parent, octant), and each internal node's children by octant, marked
+// in child_mask (zeroed beforehand) and listed in its kMaxChildren child_slots.
+// `totals` holds kMaxCooperativeBlocks words; `barrier` is zero at the start.
 constexpr uint32_t kMaxChildren = 8;
-cudaError_t launch_layout_write(const unsigned long long *codes, uint32_t n, uint32_t leaf_cap,
-                                const uint32_t *offsets, uint32_t node_capacity,
-                                DeviceNode *nodes, uint32_t *child_mask, uint32_t *child_slots,
-                                TreeMeta *meta, unsigned *status, cudaStream_t stream);
+cudaError_t launch_layout(const unsigned long long *codes, uint32_t n, uint32_t leaf_cap,
+                          uint32_t *offsets, uint32_t *totals, uint32_t node_capacity,
+                          DeviceNode *nodes, uint32_t *child_mask, uint32_t *child_slots,
+                          TreeMeta *meta, unsigned *barrier, unsigned *status,
+                          cudaStream_t stream);
 
 // Moments bottom-up (mass, centre of mass, quadrupole, acceptance radius) and
 // the leaf-relative FP32 source positions the walk reads.

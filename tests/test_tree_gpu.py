@@ -92,6 +92,24 @@ def test_ragged_sizes_and_parameters_against_oracle(b200, restatement, n, leaf, 
         assert a.tolist() == [[0.0, 0.0, 0.0]]
 
 
+# 2,048 keys make a sort tile; 1,212,417 make one more than the ordering's CTAs.
+@pytest.mark.parametrize("n", [2047, 2048, 2049, 151553, 1212417])
+def test_ordering_and_layout_at_the_edges_of_tiles(b200, restatement, n):
+    from orrery_b200 import initial_conditions as ic
+    d = ic.plummer_sphere(n, seed=n)
+    x, y, z, m = _xyzm(d)
+    t_ref, codes_ref, idx_ref = restatement.tree(x, y, z, m, 1.0, 16, True)
+    s = b200.B200TreeSolver(0.02, 1.0, 16, True)
+    for _ in range(2):  # the second evaluation starts from the first one's scratch
+        s.evaluate((x, y, z), m)
+        codes, idx, _, _ = s.order(n)
+        assert np.array_equal(codes, codes_ref) and np.array_equal(idx.astype(np.uint64), idx_ref)
+        reals, nidx, quads, leaves, depth = s.tree()
+        assert np.array_equal(nidx, t_ref.idx) and np.array_equal(reals, t_ref.reals)
+        assert np.array_equal(quads, t_ref.quads)
+        assert (leaves, depth) == (t_ref.leaf_count, t_ref.depth)
+
+
 # 65,536, 131,072 and 262,144 targets are the most that 8, 4 and 2 warps per
 # group of 32 take; a second group starts at 33.
 @pytest.mark.parametrize("n,quad", [(31, True), (32, False), (33, True), (65536, True),
