@@ -170,8 +170,7 @@ int ob_morton_order_noalloc(uint64_t n, const double *x, const double *y, const 
                             void *stream);
 
 /* Tile shape of the direct kernels: threads per CTA, targets per thread, the
- * number of CTAs (one thread-block cluster) that split the sources of a
- * target tile, and the number of thread groups of a CTA that split each
+ * number of CTAs (parts) that split the sources of a target tile, and the number of thread groups of a CTA that split each
  * staged tile's sources (each group serves the CTA's targets; 0 reads as 1).
  * A CTA holds threads * targets_per_thread / groups targets. No reference
  * counterpart: the reference picks one block size

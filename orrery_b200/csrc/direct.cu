@@ -956,6 +956,9 @@ static double direct_cost(const DirectConfig &c, double per_pair, uint32_t n, ui
     return cost;
 }
 
+// Memory the parts' sums may take (a large system gains nothing from parts).
+constexpr size_t kPartsBytes = size_t{64} << 20;
+
 DirectConfig direct_default_config(uint32_t n, bool split, int sm_count) {
     // The cheapest of a few 256-thread shapes by the estimate above, whose
     // constants are fitted to sweeps from 1,000 to 262,144 particles on B200.
@@ -986,6 +989,9 @@ DirectConfig direct_default_config(uint32_t n, bool split, int sm_count) {
             c.targets_per_thread = shapes[k].targets;
             c.groups = shapes[k].groups;
             c.split = parts;
+            if (direct_partial_doubles(n, c) * sizeof(double) > kPartsBytes) {
+                continue;
+            }
             const double cost = direct_cost(c, shapes[k].per_pair, n, sms);
             if (best_cost == 0.0 || cost < best_cost) {
                 best = c;

@@ -288,3 +288,28 @@ def test_device_pointer_entry_point(b200, golden_plummer):
     torch.cuda.synchronize()
     a = torch.stack(outs, dim=1).cpu().numpy()
     assert np.array_equal(a, g["direct_eps0.01"])
+
+
+# Parts of a target tile added through a cluster (the grid fits 2 x 148 CTAs) or
+# through memory (it does not), ragged last tiles and pairs; the same sums again
+# on the next launch, which starts from the words the first one left.
+@pytest.mark.parametrize("precision", ["fp32", "split"])
+@pytest.mark.parametrize("n,shape", [(513, None), (2367, (256, 2, 4, 8)), (2369, (256, 2, 8, 8)),
+                                     (4097, (256, 4, 8, 8)), (9473, (256, 4, 4, 8)),
+                                     (9473, (128, 2, 4, 1)), (10007, None), (12289, None)])
+def test_parts_are_added_in_order_wherever_they_meet(b200, restatement, precision, n, shape):
+    from orrery_b200 import initial_conditions as ic
+    d = ic.plummer_sphere(n, seed=n)
+    x, y, z, m = _xyzm(d)
+    exact, _ = restatement.direct(x, y, z, m, 0.05)
+    s = b200.B200DirectSolver(0.05, precision)
+    if shape is not None:
+        s.set_shape(n, shape)
+    a = s.evaluate((x, y, z), m)
+    err = relative_errors(a, exact)
+    if precision == "fp32":
+        assert err.max() < FP32_WORST and np.sqrt(np.mean(err ** 2)) < FP32_RMS
+    else:
+        assert np.median(err) < SPLIT_MEDIAN and err.max() < 1e-5
+    for _ in range(2):
+        assert np.array_equal(s.evaluate((x, y, z), m), a)
