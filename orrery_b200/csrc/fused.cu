@@ -18,19 +18,21 @@
 //      positions and masses into buffer s % 2 (already in the pair layout
 //      the pair loop reads) and then raises the CTA's ready word to this
 //      substep's number;
-//   B. every warp copies its share of the sources from buffer s % 2 into
-//      shared memory, each 32-source chunk by one bulk copy once the ready
-//      word of the CTA that wrote it has reached this substep (no grid-wide
-//      barrier: a warp waits only for the chunks it copies; the CTA waits on
-//      an mbarrier for the bytes of all of them);
+//   B. every warp copies its own slice of the sources from buffer s % 2 into
+//      shared memory by one bulk copy, once the ready words of the CTAs that
+//      wrote it have reached this substep (no grid-wide barrier: a warp waits,
+//      on its own mbarrier, only for the slice it sums; with one mbarrier for
+//      the whole CTA a 64-particle step took 3.0 us,
+//      now 2.4, a 1,000-particle one 5.5, now 4.7, a 5,500-particle one 28.4,
+//      now 25.0; 4,096, bound by the pair loop's FP32 pipe, 11.9 and 11.8);
 //   C. the CTA evaluates its targets' accelerations: FP32 pair arithmetic
 //      two sources per packed FP32x2 instruction, each warp's slice summed
 //      in FP32, the W slices added in FP64 in slice order by warp 0.
 // Double buffering is safe with per-CTA words: a CTA writes buffer s % 2
 // again only at substep s + 2, after its forces of substep s + 1, which need
-// every CTA's chunk of substep s + 1, which each CTA publishes only after its
-// copies of buffer s % 2 have landed. After the last substep warp 0 gives the
-// targets the closing kick and writes their state back.
+// every CTA's chunk of substep s + 1, which each CTA publishes only after all
+// its warps' copies of buffer s % 2 have landed and been summed. After the last
+// substep warp 0 gives the targets the closing kick and writes their state back.
 //
 // Ready words count substeps across launches (the host passes the count so
 // far, `epoch`, and clears the words together with it); waits are bounded
@@ -56,8 +58,8 @@ constexpr uint32_t kFusedMaxWarps = 32;
 // Source padding: a whole number of pairs per slice for 16 or 32 warps.
 constexpr uint32_t kFusedGroup = 2 * kFusedMaxWarps;
 constexpr size_t kFusedSmemCap = 200u * 1024u; // dynamic shared memory (sources)
-// Every warp's chunks have their ready words polled by one lane each.
-static_assert(kFusedSmemCap / 16u / 32u / 16u <= 32u, "at most 32 chunks per warp");
+// The ready words of a warp's slice are polled by one lane each.
+static_assert(kFusedSmemCap / 16u / 32u / 16u + 2u <= 32u, "at most 32 writers per slice");
 // Ready words one 128-byte line apart: polls of different CTAs' words then go
 // to different L2 lines instead of queueing on a few.
 constexpr uint32_t kReadyStride = 32;
@@ -137,8 +139,9 @@ __global__ void __launch_bounds__(WARPS * 32)
     extern __shared__ __align__(16) float4 src[]; // pairs: (x0 x1 y0 y1) (z0 z1 m0 m1)
     __shared__ double partial[WARPS][3][kFusedTargets];
     __shared__ double state[9][kFusedTargets]; // x y z vx vy vz ax ay az of the CTA's targets
+    __shared__ float target_of[4][kFusedTargets]; // x y z m of the CTA's targets, FP32
     __shared__ int stop;
-    __shared__ __align__(8) uint64_t loaded; // the substep's source chunks have landed
+    __shared__ __align__(8) uint64_t loaded[WARPS]; // the warp's sources have landed
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     const uint32_t i = blockIdx.x * kFusedTargets + lane; // this lane's target in every warp
     const bool mine = i < g.n;
@@ -148,17 +151,25 @@ __global__ void __launch_bounds__(WARPS * 32)
         for (int k = 0; k < 9; ++k) {
             state[k][lane] = mine ? global_state[k][i] : 0.0;
         }
+        for (int k = 0; k < 3; ++k) {
+            target_of[k][lane] = 0.0f;
+        }
         mass = mine ? __double2float_rn(g.m[i]) : 0.0f;
     }
     if (threadIdx.x == 0) {
         stop = 0;
-        mbar_init(&loaded, 1);
+        for (uint32_t w = 0; w < WARPS; ++w) {
+            mbar_init(&loaded[w], 1);
+        }
         fence_barrier_init();
     }
     __syncthreads();
     const uint32_t blocks = gridDim.x;
-    const uint32_t chunks = g.padded / 32u; // 32-source chunks, padding included
     const uint32_t slice = g.padded / 2u / WARPS; // pairs per warp
+    const uint32_t p0 = warp * slice, p1 = p0 + slice;
+    // The CTAs that publish this warp's slice: 16 pairs each, one lane polls each.
+    const uint32_t writer = p0 / 16u + lane;
+    const bool polling = writer < blocks && writer * 16u < p1;
     const float2 e2 = f2(g.eps2, g.eps2);
     uint32_t s = 0;
     for (; s < g.substeps; ++s) {
@@ -167,6 +178,7 @@ __global__ void __launch_bounds__(WARPS * 32)
         float4 *buf = (s & 1u) != 0u ? g.buf1 : g.buf0;
         // A. Kick and drift this CTA's targets, publish their FP32 copy.
         if (warp == 0) {
+            target_of[3][lane] = mass;
             if (mine) {
                 double vx = state[3][lane], vy = state[4][lane], vz = state[5][lane];
                 const double ax = state[6][lane], ay = state[7][lane], az = state[8][lane];
@@ -192,10 +204,15 @@ __global__ void __launch_bounds__(WARPS * 32)
                 // layout the pair loop reads, so that chunks copy as they are.
                 float *lo = reinterpret_cast<float *>(&buf[2u * (i >> 1)]) + (i & 1u);
                 float *hi = reinterpret_cast<float *>(&buf[2u * (i >> 1) + 1u]) + (i & 1u);
-                lo[0] = __double2float_rn(x);
-                lo[2] = __double2float_rn(y);
-                hi[0] = __double2float_rn(z);
+                const float fx = __double2float_rn(x), fy = __double2float_rn(y),
+                            fz = __double2float_rn(z);
+                lo[0] = fx;
+                lo[2] = fy;
+                hi[0] = fz;
                 hi[2] = mass;
+                target_of[0][lane] = fx;
+                target_of[1][lane] = fy;
+                target_of[2][lane] = fz;
             }
             asm volatile("fence.proxy.async.global;" ::: "memory");
             __threadfence();
@@ -204,61 +221,44 @@ __global__ void __launch_bounds__(WARPS * 32)
                 store_release(&g.ready[blockIdx.x * kReadyStride], target);
             }
         }
-        // B. Sources into shared memory, chunk q = sources 32q .. 32q + 31
-        // (512 bytes; zero-mass padding at the origin past N, zeroed once on
-        // the host and never written), once the CTA that wrote each chunk has
-        // published it. Warp w copies chunks w, w + W, ...: lane k polls the
-        // ready word of the warp's k-th chunk (at most 32) and then starts
-        // its bulk copy, completing on `loaded`, whose byte count thread 0
-        // posts for the substep. A chunk whose wait ran out is copied all
-        // the same, so that the barrier completes and no copy is left in
-        // flight; the substep is then abandoned.
-        if (threadIdx.x == 0) {
-            mbar_arrive_expect_tx(&loaded, g.padded * 16u);
-        }
-        {
-            const uint32_t q = warp + WARPS * lane;
-            const bool copies = q < chunks;
-            const bool polling = copies && q < blocks;
-            for (uint32_t polls = 0;; ++polls) {
-                const bool behind =
-                    polling && !reached(load_acquire(&g.ready[q * kReadyStride]), target);
-                if (!__any_sync(0xffffffffu, behind)) {
-                    break;
-                }
-                if (polls >= g.poll_limit) {
-                    if (lane == 0) {
-                        atomicOr(g.status, kStatusTimeout);
-                        stop = 1;
-                    }
-                    break;
-                }
+        __syncthreads(); // the targets are in place; the last substep's readers are done
+        // B. The warp's slice of the sources into shared memory by one bulk copy
+        // (zero-mass padding at the origin past N, zeroed once on the host and
+        // never written), once the CTAs that write it have published it: lane k
+        // polls the ready word of the k-th of them (at most 27). Warps wait for
+        // their own slices only, so the first to arrive are summed while others
+        // are on their way. Where a wait ran out the slice is copied all the
+        // same, so that the barrier completes and no copy is left in flight; the
+        // substep is then abandoned.
+        for (uint32_t polls = 0;; ++polls) {
+            const bool behind =
+                polling && !reached(load_acquire(&g.ready[writer * kReadyStride]), target);
+            if (!__any_sync(0xffffffffu, behind)) {
+                break;
             }
-            if (copies) {
-                // The chunk's generic-proxy writes (acquired above) before
-                // the async-proxy read; this CTA's reads of the previous
-                // substep's sources before the async-proxy write.
-                asm volatile("fence.proxy.async.global;" ::: "memory");
-                fence_proxy_async_shared();
-                bulk_copy_g2s(&src[32u * q], &buf[32u * q], 512u, &loaded);
+            if (polls >= g.poll_limit) {
+                if (lane == 0) {
+                    atomicOr(g.status, kStatusTimeout);
+                    stop = 1;
+                }
+                break;
             }
         }
-        if (!mbar_wait_bounded(&loaded, s & 1u, g.status)) {
+        __syncwarp(); // the lanes' acquires before lane 0's copy
+        if (lane == 0) {
+            // The slice's generic-proxy writes (acquired above) before the
+            // async-proxy read; this warp's reads of the previous substep's
+            // sources before the async-proxy write.
+            asm volatile("fence.proxy.async.global;" ::: "memory");
+            fence_proxy_async_shared();
+            mbar_arrive_expect_tx(&loaded[warp], slice * 32u);
+            bulk_copy_g2s(&src[2u * p0], &buf[2u * p0], slice * 32u, &loaded[warp]);
+        }
+        // C. This CTA's targets against the warp's slice.
+        const float tx = target_of[0][lane], ty = target_of[1][lane], tz = target_of[2][lane];
+        const float tm = target_of[3][lane];
+        if (!mbar_wait_bounded(&loaded[warp], s & 1u, g.status)) {
             stop = 1;
-        }
-        __syncthreads();
-        if (stop != 0) {
-            break; // every thread reads the same word after the barrier
-        }
-        // C. This CTA's targets against every source.
-        float tx = 0.0f, ty = 0.0f, tz = 0.0f, tm = 0.0f;
-        if (mine) {
-            const float4 q0 = src[2u * (i >> 1)], q1 = src[2u * (i >> 1) + 1u];
-            const bool odd = (i & 1u) != 0u;
-            tx = odd ? q0.y : q0.x;
-            ty = odd ? q0.w : q0.z;
-            tz = odd ? q1.y : q1.x;
-            tm = odd ? q1.w : q1.z;
         }
         // With softening the target's own entry adds exactly zero (d = 0)
         // unless m / eps^3 overflows FP32; then the warp skips it by index.
@@ -267,7 +267,6 @@ __global__ void __launch_bounds__(WARPS * 32)
         const bool skip_self = __any_sync(0xffffffffu, mine && !(fabsf(self_term) < 3.0e38f));
         const float2 ntx = f2(-tx, -tx), nty = f2(-ty, -ty), ntz = f2(-tz, -tz);
         float2 sx = f2(0.0f, 0.0f), sy = sx, sz = sx;
-        const uint32_t p0 = warp * slice, p1 = p0 + slice;
         // The warp-uniform choice is made once, outside the pair loop.
         if (skip_self) {
             pair_slice<true>(src, p0, p1, i, ntx, nty, ntz, e2, sx, sy, sz);
@@ -277,20 +276,25 @@ __global__ void __launch_bounds__(WARPS * 32)
         partial[warp][0][lane] = static_cast<double>(sx.x) + static_cast<double>(sx.y);
         partial[warp][1][lane] = static_cast<double>(sy.x) + static_cast<double>(sy.y);
         partial[warp][2][lane] = static_cast<double>(sz.x) + static_cast<double>(sz.y);
-        // The sources are read and the partials written: warp 0 adds the
-        // slices while the other warps go on to the next substep's loads,
-        // which wait for warp 0's next publication.
+        // The partials are written: warp 0 adds the slices (even and odd ones
+        // apart, which halves the chain) and goes on to the next kick, for which
+        // the other warps wait.
         __syncthreads();
+        if (stop != 0) {
+            break; // every thread reads the same word after the barrier
+        }
         if (warp == 0) {
-            double a[3] = {0.0, 0.0, 0.0};
-            for (uint32_t w = 0; w < WARPS; ++w) {
+            double a[3] = {0.0, 0.0, 0.0}, b[3] = {0.0, 0.0, 0.0};
+#pragma unroll 8
+            for (uint32_t w = 0; w < WARPS; w += 2) {
                 for (int k = 0; k < 3; ++k) {
                     a[k] += partial[w][k][lane];
+                    b[k] += partial[w + 1u][k][lane];
                 }
             }
-            state[6][lane] = a[0];
-            state[7][lane] = a[1];
-            state[8][lane] = a[2];
+            state[6][lane] = a[0] + b[0];
+            state[7][lane] = a[1] + b[1];
+            state[8][lane] = a[2] + b[2];
         }
     }
     // The closing kick of the last substep, and the state back to HBM (as
