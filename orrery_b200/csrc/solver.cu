@@ -125,7 +125,7 @@ DirectConfig Solver::direct_config(uint32_t n) {
     return c;
 }
 
-DirectParts Solver::reserve_parts(uint32_t n, const DirectConfig &config, cudaStream_t stream) {
+DirectParts Solver::reserve_parts(uint32_t n, const DirectConfig &config) {
     if (direct_uses_cluster(n, config)) {
         return {};
     }
@@ -133,9 +133,16 @@ DirectParts Solver::reserve_parts(uint32_t n, const DirectConfig &config, cudaSt
         ++generation_;
     }
     if (part_arrived_.reserve(direct_arrival_words(n, config))) {
-        check(cudaMemsetAsync(part_arrived_.data(), 0, part_arrived_.bytes(), stream),
-              "clearing the arrival words");
         ++generation_;
+        // Cleared here and now, on the solver's own stream: on the caller's the
+        // clear may become a node of a graph that is never launched.
+        const cudaError_t err =
+            cudaMemsetAsync(part_arrived_.data(), 0, part_arrived_.bytes(), stream_);
+        const cudaError_t done = err == cudaSuccess ? cudaStreamSynchronize(stream_) : err;
+        if (done != cudaSuccess) {
+            part_arrived_.release(); // never used uncleared
+            check(done, "clearing the arrival words");
+        }
     }
     return {part_sums_.data(), part_arrived_.data()};
 }
@@ -160,7 +167,7 @@ void Solver::evaluate_direct(uint32_t n, const double *x, const double *y, const
     if (split && lo_.reserve(2ull * padded)) {
         ++generation_;
     }
-    const DirectParts parts = reserve_parts(n, config, stream);
+    const DirectParts parts = reserve_parts(n, config);
     check(pack_sources(x, y, z, m, n, padded, hi_.data(), split ? lo_.data() : nullptr, stream),
           "packing sources");
     record(ordered, stream, external);
@@ -213,7 +220,7 @@ double Solver::autotune(uint32_t n, DirectConfig &chosen) {
         }
         const uint32_t padded = direct_padded_count(n, c);
         hi_.reserve((split ? 2ull : 1ull) * padded);
-        const DirectParts parts = reserve_parts(n, c, stream_);
+        const DirectParts parts = reserve_parts(n, c);
         if (split) {
             lo_.reserve(2ull * padded);
         }

@@ -91,8 +91,9 @@ private:
                          bool external);
 
     // Where the parts of a split source range leave their sums (kept between
-    // evaluations; empty while a cluster adds them).
-    DirectParts reserve_parts(uint32_t n, const DirectConfig &config, cudaStream_t stream);
+    // evaluations; empty while a cluster adds them). The arrival words are clear
+    // when it returns, whether or not the caller's stream is being captured.
+    DirectParts reserve_parts(uint32_t n, const DirectConfig &config);
 
     ob_solver_params params_;
     int sm_count_ = 148;

@@ -12,6 +12,8 @@ from __future__ import annotations
 import numpy as np
 import pytest
 
+from conftest import relative_errors
+
 pytestmark = pytest.mark.gpu
 
 KEYS = ("x", "y", "z", "vx", "vy", "vz", "ax", "ay", "az")
@@ -339,3 +341,43 @@ def test_blocks_of_destroyed_objects_serve_new_ones_from_several_threads(b200, r
     for t in threads:
         t.join()
     assert not failures
+
+
+def _leave_nonzero_blocks(b200):
+    # Solvers over host arrays leave small device blocks full of coordinates to
+    # the objects that come after them.
+    from orrery_b200 import initial_conditions as ic
+    for n in (9, 17, 25, 33, 49) * 30:
+        d = ic.plummer_sphere(n, seed=n)
+        b200.B200DirectSolver(0.01, "fp64").evaluate((d["x"], d["y"], d["z"]), d["m"])
+
+
+# Sizes whose parts are added through memory: a system's first evaluation may
+# stand in a graph that is captured and not launched.
+@pytest.mark.parametrize("first", ["step_host", "restore and profile", "restore and step_kernels"])
+@pytest.mark.parametrize("precision,n", [("fp32", 10007), ("fp32", 20011), ("split", 10007),
+                                         ("split", 20011)])
+def test_parts_start_clear_whatever_a_system_does_first(b200, restatement, tmp_path, precision, n,
+                                                        first):
+    from orrery_b200 import initial_conditions as ic
+    d = ic.plummer_sphere(n, seed=n)
+    state = {k: np.array(d[k]) for k in ("x", "y", "z", "vx", "vy", "vz", "m")}
+    state.update(ax=np.full(n, 1e3), ay=np.full(n, 1e3), az=np.full(n, 1e3))
+    _leave_nonzero_blocks(b200)
+    s = b200.DeviceSystem(n, 0.02, precision=precision)
+    if first == "step_host":
+        s.step_host(state, 1e-4, 1, "vv")
+    else:
+        b200.write_checkpoint(tmp_path / "c", 0, state)
+        s.read_checkpoint(tmp_path / "c")
+        if first == "restore and profile":
+            s.profile(1)
+        else:
+            s.step_kernels(1e-3, "vv")
+        s.step(1e-4, 1, "vv")
+        state.update(s.state())
+    exact, _ = restatement.direct(state["x"], state["y"], state["z"], d["m"], 0.02)
+    a = np.stack([state["ax"], state["ay"], state["az"]], axis=1)
+    err = relative_errors(a, exact)
+    # The bounds of the forms' own tests (test_direct_gpu.py).
+    assert err.max() < (2e-4 if precision == "fp32" else 1e-5)
