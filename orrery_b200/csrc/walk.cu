@@ -74,11 +74,11 @@
 // particles (quadrupoles, two warps per group) the FMA pipe is 48 % busy and
 // 60 % of issue slots are used. Walk times, before (one warp per group, one
 // stack item per node) and after: 10,000 Plummer particles without quadrupoles
-// 360 -> 117 us; 100,000 collision particles 756 -> 666 us; 200,000 1.40 -> 1.32 ms;
-// 2,000,000 14.79 -> 14.42 ms. Relative error against 64 bits (2-norm): 10,000
-// 7.7e-8 -> 5.2e-8, 200,000 4.2e-8 -> 4.3e-8, 2,000,000 3.9e-8 -> 4.1e-8 (the
-// families of a batch pull the same way, so its FP32 partial sums are larger). Groups of 64 targets (two per lane) halve the
-// traversal but measured no faster at any size (2M 14.60 ms).
+// 367 -> 119 us; 100,000 collision particles 752 -> 672 us; 200,000 1.41 -> 1.33
+// ms; 2,000,000 14.89 -> 14.72 ms. Relative error against the FP64 walk (2-norm):
+// 10,000 8.1e-8 -> 5.3e-8, 200,000 3.89e-8 -> 3.78e-8, 2,000,000 3.73e-8 ->
+// 3.70e-8 (flush_cells says how the cells are summed). Groups of 64 targets (two
+// per lane) halve the traversal but measured no faster at any size.
 #include <algorithm>
 #include <atomic>
 
@@ -102,8 +102,8 @@ constexpr uint32_t kFamilies = 4;
 constexpr uint32_t kStackCap = 256;
 constexpr uint32_t kCellCap = 48;
 constexpr uint32_t kLeafCap = 40;
-// Cells summed in one FP32 chain.
-constexpr uint32_t kCellBlock = 16;
+// Cells of a block, two FP32 chains of half as many terms (flush_cells).
+constexpr uint32_t kCellBlock = 8;
 // Leaves summed in FP32 before their sums are folded into FP64.
 constexpr uint32_t kLeafFold = 8;
 // Staged cell fields, as quads of packed pairs: quad f of pair p holds
@@ -410,10 +410,19 @@ __device__ __forceinline__ void cell_pair(const WarpSpace &ws, uint32_t p, float
 }
 
 // Evaluates the staged cells: every lane sums every cell for its target (zero
-// outside the cell's mask), two cells per FP32x2 instruction, four per loop
-// step (the batch is padded with neutral entries to a multiple of four).
-// Each lane holds its target relative to G, so the offset to a cell is one
-// subtraction.
+// outside the cell's mask), two cells per FP32x2 instruction (an odd count is
+// padded with one neutral entry). Each lane holds its target relative to G, so
+// the offset to a cell is one subtraction.
+//
+// The cells of a family follow one another and pull the same way, so a chain's
+// partial sums grow along it and its FP32 rounding with them. Quadrupole cells
+// are summed in blocks of eight: 2-norm error against the FP64 walk at 200,000
+// and 2,000,000 particles (collision) 3.78e-8 and 3.70e-8, in blocks of sixteen
+// 3.91e-8 and 3.85e-8, one chain over cells in pre-order 3.89e-8 and 3.73e-8
+// (walk 14.7, 14.5 and 14.9 ms at 2,000,000). Monopole cells, whose terms are
+// shorter, go to two chains by turns, which meet in FP64: 1,000,000 Plummer
+// particles 3.61e-8 and 4.62 ms, in blocks of eight 3.74e-8 and 4.79 ms, of
+// sixteen 3.77e-8 and 4.70 ms, one pre-order chain 3.65e-8 and 4.70 ms.
 template <bool QUAD>
 __device__ __forceinline__ void flush_cells(WarpSpace &ws, uint32_t count, float2 ntx, float2 nty,
                                             float2 ntz, float2 eps2, uint32_t lane_bit,
@@ -427,23 +436,41 @@ __device__ __forceinline__ void flush_cells(WarpSpace &ws, uint32_t count, float
         ws.cell_mask[count] = 0u;
     }
     __syncwarp();
-    // Blocks of cells are summed by themselves and then added to the batch's
-    // sums: shorter FP32 chains, smaller rounding.
-    float2 sx = f2(0.0f, 0.0f), sy = sx, sz = sx;
-    for (uint32_t from = 0; from < count; from += kCellBlock) {
-        const uint32_t to = min(from + kCellBlock, count);
-        float2 bx = f2(0.0f, 0.0f), by = bx, bz = bx;
-        for (uint32_t j = from; j < to; j += 2) {
-            cell_pair<QUAD>(ws, j >> 1, ntx, nty, ntz, eps2, lane_bit, bx, by, bz);
+    if constexpr (QUAD) {
+        float2 sx = f2(0.0f, 0.0f), sy = sx, sz = sx;
+        for (uint32_t from = 0; from < count; from += kCellBlock) {
+            const uint32_t to = min(from + kCellBlock, count);
+            float2 bx = f2(0.0f, 0.0f), by = bx, bz = bx;
+            for (uint32_t j = from; j < to; j += 2) {
+                cell_pair<true>(ws, j >> 1, ntx, nty, ntz, eps2, lane_bit, bx, by, bz);
+            }
+            sx = __fadd2_rn(sx, bx);
+            sy = __fadd2_rn(sy, by);
+            sz = __fadd2_rn(sz, bz);
         }
-        sx = __fadd2_rn(sx, bx);
-        sy = __fadd2_rn(sy, by);
-        sz = __fadd2_rn(sz, bz);
+        __syncwarp();
+        acc_x += static_cast<double>(sx.x) + static_cast<double>(sx.y);
+        acc_y += static_cast<double>(sy.x) + static_cast<double>(sy.y);
+        acc_z += static_cast<double>(sz.x) + static_cast<double>(sz.y);
+    } else {
+        const uint32_t pairs = (count + 1u) >> 1;
+        float2 sx = f2(0.0f, 0.0f), sy = sx, sz = sx, bx = sx, by = sx, bz = sx;
+#pragma unroll 1
+        for (uint32_t p = 0; p + 1u < pairs; p += 2u) {
+            cell_pair<false>(ws, p, ntx, nty, ntz, eps2, lane_bit, sx, sy, sz);
+            cell_pair<false>(ws, p + 1u, ntx, nty, ntz, eps2, lane_bit, bx, by, bz);
+        }
+        if ((pairs & 1u) != 0u) {
+            cell_pair<false>(ws, pairs - 1u, ntx, nty, ntz, eps2, lane_bit, sx, sy, sz);
+        }
+        __syncwarp();
+        acc_x += (static_cast<double>(sx.x) + static_cast<double>(sx.y)) +
+                 (static_cast<double>(bx.x) + static_cast<double>(bx.y));
+        acc_y += (static_cast<double>(sy.x) + static_cast<double>(sy.y)) +
+                 (static_cast<double>(by.x) + static_cast<double>(by.y));
+        acc_z += (static_cast<double>(sz.x) + static_cast<double>(sz.y)) +
+                 (static_cast<double>(bz.x) + static_cast<double>(bz.y));
     }
-    __syncwarp();
-    acc_x += static_cast<double>(sx.x) + static_cast<double>(sx.y);
-    acc_y += static_cast<double>(sy.x) + static_cast<double>(sy.y);
-    acc_z += static_cast<double>(sz.x) + static_cast<double>(sz.y);
 }
 
 // Evaluates the queued leaves: for each, every lane sums its particles for its

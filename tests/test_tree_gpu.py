@@ -131,6 +131,22 @@ def test_every_number_of_warps_per_group_gives_the_oracle_s_counts(b200, restate
     assert np.array_equal(a, again)  # the warps' sums are added in a fixed order
 
 
+# The bounds are what one FP32 chain over the cells in pre-order gave on these
+# inputs (the sums have a fixed order, so the errors do not vary): families, which
+# pull the same way, must not make the walk's rounding larger.
+@pytest.mark.parametrize("model,n,quad,angle,bound", [("collision", 300000, True, 0.5, 3.71e-8),
+                                                      ("plummer", 700000, False, 0.6, 4.30e-8),
+                                                      ("plummer", 700000, True, 0.6, 4.46e-8)])
+def test_families_of_cells_do_not_grow_the_walk_s_rounding(b200, model, n, quad, angle, bound):
+    from orrery_b200 import initial_conditions as ic
+    d = (ic.galaxy_collision(n, softening=0.02, seed=31) if model == "collision"
+         else ic.plummer_sphere(n, seed=9))
+    x, y, z, m = _xyzm(d)
+    a = b200.B200TreeSolver(0.02, angle, 32, quad).evaluate((x, y, z), m)
+    exact = b200.B200TreeSolver(0.02, angle, 32, quad, "fp64").evaluate((x, y, z), m)
+    assert np.linalg.norm(a - exact) < bound * np.linalg.norm(exact)
+
+
 # --------------------------------------------------------------------------
 # The FP64 parity mode: forces equal to BarnesHutSolver's bit for bit
 # --------------------------------------------------------------------------
