@@ -345,6 +345,20 @@ Batch::Batch(uint32_t systems, const uint64_t *counts, const double *softening_s
 
 Batch::~Batch() {
     drop_graph();
+    // Every array is used on the batch's stream alone.
+    if (stream_ != nullptr && finished(stream_)) {
+        state_.keep();
+        hi_.keep();
+        lo_.keep();
+        eps2_.keep();
+        items_.keep();
+        side_items_.keep();
+        groups_.keep();
+        partial_.keep();
+        queue_.keep();
+        status_.keep();
+        terms_.keep();
+    }
     if (stream_ != nullptr && owns_stream_) {
         cudaStreamDestroy(stream_);
     }

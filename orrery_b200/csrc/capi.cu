@@ -83,6 +83,13 @@ System::System(const ob_solver_params &params, uint32_t n, cudaStream_t stream)
 
 System::~System() {
     drop_graph();
+    // Everything but the state (whose addresses callers may hold) is used on the
+    // system's own stream alone.
+    if (stream_ != nullptr && finished(stream_)) {
+        solver_->keep_blocks();
+        terms_.keep();
+        rk4_.keep();
+    }
     for (auto e : marks_) {
         cudaEventDestroy(e);
     }

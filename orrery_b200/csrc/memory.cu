@@ -6,6 +6,11 @@
 // every time. Blocks of destroyed objects are therefore kept, at most
 // kKeptBytes and kKeptBlocks of them in the process, and given back to the
 // device when that is exceeded or when an allocation fails.
+//
+// Nothing here waits: an owner keeps a block once its own streams have finished
+// with it, and frees (cudaFree, which waits by itself) what a caller's stream or
+// pointer may still use. A wait for the whole device in a destructor would
+// invalidate every graph capture under way in other threads.
 #include <algorithm>
 #include <mutex>
 #include <vector>
@@ -100,12 +105,7 @@ void *take_device_block(size_t bytes, size_t &got, int &device) {
 }
 
 void keep_device_block(void *ptr, size_t bytes, int device) noexcept {
-    int current = -1;
-    // As cudaFree does, wait for the device: work on any stream may still use
-    // the block, and its next owner must not.
-    if (bytes > kKeptBytes / 4 || cudaGetDevice(&current) != cudaSuccess || current != device ||
-        cudaDeviceSynchronize() != cudaSuccess) {
-        cudaGetLastError();
+    if (bytes > kKeptBytes / 4) {
         cudaFree(ptr);
         return;
     }

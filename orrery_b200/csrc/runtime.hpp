@@ -61,8 +61,8 @@ int set_error(int code, const std::string &message);
 // A device block of at least `bytes` on the current device: one kept from a
 // destroyed object, or newly allocated (memory.cu). Its contents are undefined.
 void *take_device_block(size_t bytes, size_t &got, int &device);
-// Keeps a block for the next object (bounded; else frees it), once the device
-// has finished what may use it.
+// Keeps a block for the next object (bounded; else frees it). Nothing enqueued
+// on the device may still use it.
 void keep_device_block(void *ptr, size_t bytes, int device) noexcept;
 
 // Owning device allocation that grows on demand and never shrinks, the
@@ -81,11 +81,7 @@ public:
         }
         return *this;
     }
-    ~DeviceArray() {
-        if (ptr_ != nullptr) {
-            keep_device_block(ptr_, block_bytes_, device_);
-        }
-    }
+    ~DeviceArray() { release(); }
 
     // Returns true when the storage moved (callers holding the old pointer,
     // such as captured graphs, must refresh).
@@ -101,6 +97,15 @@ public:
     void release() noexcept {
         if (ptr_ != nullptr) {
             cudaFree(ptr_);
+        }
+        ptr_ = nullptr;
+        count_ = 0;
+    }
+    // Releases the storage to the next object's use: for owners that know that
+    // nothing enqueued on the device may still use it.
+    void keep() noexcept {
+        if (ptr_ != nullptr) {
+            keep_device_block(ptr_, block_bytes_, device_);
         }
         ptr_ = nullptr;
         count_ = 0;
@@ -122,6 +127,15 @@ private:
     size_t block_bytes_ = 0; // of the whole block, which may exceed count_ values
     int device_ = 0;
 };
+
+// True once all work enqueued on `stream` has finished.
+inline bool finished(cudaStream_t stream) noexcept {
+    if (cudaStreamSynchronize(stream) == cudaSuccess) {
+        return true;
+    }
+    cudaGetLastError();
+    return false;
+}
 
 // Records `event` on `stream`; `external` makes it a real event-record node
 // when the stream is being captured into a graph.

@@ -76,7 +76,30 @@ Solver::Solver(const ob_solver_params &params) : params_(corrected(params)) {
     }
 }
 
+void Solver::keep_blocks() noexcept {
+    hi_.keep();
+    lo_.keep();
+    part_sums_.keep();
+    part_arrived_.keep();
+    staging_.keep();
+    status_.keep();
+    if (tree_) {
+        tree_->keep_blocks();
+    }
+}
+
 Solver::~Solver() {
+    // Evaluations share these arrays, so a caller orders them whatever streams
+    // they are on, and the last one's closing event tells that all have finished.
+    // A graph that holds one may be replayed at any time: then the arrays are
+    // freed, which waits.
+    if (stream_ != nullptr && !captured_ && !open_ && finished(stream_)) {
+        if (cudaEventSynchronize(events_[4]) == cudaSuccess) {
+            keep_blocks();
+        } else {
+            cudaGetLastError();
+        }
+    }
     for (auto &e : events_) {
         if (e != nullptr) {
             cudaEventDestroy(e);
@@ -275,6 +298,15 @@ void Solver::account(uint64_t evaluations, uint64_t n) {
 void Solver::evaluate_device(uint32_t n, const double *x, const double *y, const double *z,
                              const double *m, double *ax, double *ay, double *az,
                              cudaStream_t stream, bool count, const cudaEvent_t *marks) {
+    if (!captured_ && stream != stream_) {
+        cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(stream, &capturing) != cudaSuccess) {
+            cudaGetLastError();
+            captured_ = true;
+        }
+        captured_ = captured_ || capturing != cudaStreamCaptureStatusNone;
+    }
+    open_ = true;
     const bool external = marks != nullptr;
     const cudaEvent_t *e = external ? marks : &events_[1];
     record(e[0], stream, external);
@@ -284,6 +316,7 @@ void Solver::evaluate_device(uint32_t n, const double *x, const double *y, const
         tree_->evaluate(n, x, y, z, m, ax, ay, az, status_.data(), e[1], e[2], external, stream);
     }
     record(e[3], stream, external);
+    open_ = false;
     if (count) {
         account(1, n);
     }

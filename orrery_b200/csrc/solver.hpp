@@ -80,6 +80,10 @@ public:
     // evaluation must be repeated.
     bool grew_after_overflow(cudaStream_t stream);
 
+    // Leaves the device blocks to the next objects. For the owner of the one
+    // stream that the evaluations ran on, once that stream has finished.
+    void keep_blocks() noexcept;
+
     // Times every implemented shape on synthetic sources of n particles and
     // keeps the fastest for n. Returns the time per evaluation in ms.
     double autotune(uint32_t n, DirectConfig &chosen);
@@ -106,6 +110,8 @@ private:
     ob_counts counts_{};
     std::array<cudaEvent_t, 6> events_{};
     bool timed_host_ = false;
+    bool captured_ = false; // an evaluation was captured into a caller's (or a system's) graph
+    bool open_ = false;     // an evaluation began and its closing event is not recorded (yet)
     cudaStream_t stream_ = nullptr;
     std::map<uint32_t, DirectConfig> configs_;
     uint64_t generation_ = 0;

@@ -660,6 +660,26 @@ TreePipeline::TreePipeline(const ob_solver_params &params) : params_(params) {
 
 TreePipeline::~TreePipeline() = default;
 
+void TreePipeline::keep_blocks() noexcept {
+    for (int k = 0; k < 2; ++k) {
+        keys_[k].keep();
+        perm_[k].keep();
+    }
+    scratch_.keep();
+    sorted_.keep();
+    leaf_rel_.keep();
+    node_start_.keep();
+    scan_partials_.keep();
+    nodes_.keep();
+    quads_.keep();
+    walk_records_.keep();
+    walk_index_.keep();
+    level_lists_.keep();
+    meta_.keep();
+    reduce_.keep();
+    counters_.keep();
+}
+
 uint32_t TreePipeline::nodes_for(uint32_t n) const {
     const uint64_t cap = params_.leaf_capacity < 1 ? 1 : params_.leaf_capacity;
     const uint64_t estimate = 8ull * n / cap + n / 2 + 1024;

@@ -90,6 +90,9 @@ public:
     ob_counts device_counts();
     void reset_counts();
 
+    // Leaves the device blocks to the next objects (Solver::keep_blocks).
+    void keep_blocks() noexcept;
+
     // Inspection (tests): copies the last tree and ordering to the host.
     // nodes: 5 doubles per node (mass, com xyz, r2); idx: 3 uint64 per node
     // (next, first, count); quads: 6 doubles per node or NULL.

@@ -381,3 +381,60 @@ def test_parts_start_clear_whatever_a_system_does_first(b200, restatement, tmp_p
     err = relative_errors(a, exact)
     # The bounds of the forms' own tests (test_direct_gpu.py).
     assert err.max() < (2e-4 if precision == "fp32" else 1e-5)
+
+
+def test_objects_dropped_in_one_thread_leave_another_s_captures_alone(b200, restatement):
+    # Two threads capture a step graph per timestep (FP64 and tree systems take
+    # no fused steps) while two others make solvers and systems and drop them.
+    import threading
+
+    from orrery_b200 import initial_conditions as ic
+    d = ic.plummer_sphere(700, seed=5)
+    args = [d[k] for k in ("x", "y", "z", "vx", "vy", "vz", "m")]
+    failures = []
+    stepping = [True, True]
+
+    def guarded(body):
+        try:
+            body()
+        except Exception as e:  # noqa: BLE001 - reported below, whatever it is
+            failures.append(repr(e))
+
+    def steps(k):
+        def make():
+            if k == 0:
+                return b200.DeviceSystem(700, 0.01, precision="fp64")
+            return b200.DeviceSystem(700, 0.02, b200.SOLVER_TREE, "fp64", 0.7, 8, True)
+        timesteps = [1e-4 * (1 + j % 7) for j in range(200)]
+
+        def body():
+            s = make()
+            s.set_state(*args)
+            for dt in timesteps:
+                s.step(dt, 1, "vv")
+            got.append((make, timesteps, s.state()))
+        guarded(body)
+        stepping[k] = False
+
+    def drops():
+        while any(stepping) and not failures:
+            b200.B200DirectSolver(0.01, "fp64").evaluate((d["x"], d["y"], d["z"]), d["m"])
+            s = b200.DeviceSystem(700, 0.01, precision="fp64")
+            s.set_state(*args)
+
+    got = []
+    threads = [threading.Thread(target=steps, args=(k,)) for k in range(2)]
+    threads += [threading.Thread(target=guarded, args=(drops,)) for _ in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not failures and len(got) == 2
+    for make, timesteps, end in got:  # the same steps with nothing beside them
+        s = make()
+        s.set_state(*args)
+        for dt in timesteps:
+            s.step(dt, 1, "vv")
+        alone = s.state()
+        for key in KEYS:
+            assert np.array_equal(alone[key], end[key]), key
