@@ -22,6 +22,8 @@ namespace {
 
 constexpr size_t kKeptBytes = size_t{256} << 20;
 constexpr size_t kKeptBlocks = 256;
+// Larger blocks are allocated as they are asked for and freed at once.
+constexpr size_t kLargestKept = kKeptBytes / 4;
 
 struct Block {
     void *ptr;
@@ -69,12 +71,13 @@ void *take_device_block(size_t bytes, size_t &got, int &device) {
     check(cudaGetDevice(&device), "cudaGetDevice");
     // Sizes in steps of an eighth, so that blocks fit the next object of about
     // the same size.
-    size_t step = 512;
-    while (step * 8 < bytes) {
-        step *= 2;
-    }
-    const size_t want = (bytes + step - 1) / step * step;
-    {
+    size_t want = bytes;
+    if (bytes <= kLargestKept) {
+        size_t step = 512;
+        while (step * 8 < bytes) {
+            step *= 2;
+        }
+        want = (bytes + step - 1) / step * step;
         Kept &k = kept();
         std::lock_guard<std::mutex> lock(k.mutex);
         auto best = k.blocks.end();
@@ -105,7 +108,7 @@ void *take_device_block(size_t bytes, size_t &got, int &device) {
 }
 
 void keep_device_block(void *ptr, size_t bytes, int device) noexcept {
-    if (bytes > kKeptBytes / 4) {
+    if (bytes > kLargestKept) {
         cudaFree(ptr);
         return;
     }

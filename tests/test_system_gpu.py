@@ -438,3 +438,14 @@ def test_objects_dropped_in_one_thread_leave_another_s_captures_alone(b200, rest
         alone = s.state()
         for key in KEYS:
             assert np.array_equal(alone[key], end[key]), key
+
+
+def test_a_large_block_takes_what_it_holds(b200):
+    # 80 bytes of state per particle, a little above 2^27 bytes.
+    torch = pytest.importorskip("torch")
+    n = 1677722
+    b200.DeviceSystem(64, 0.01, precision="fp64")  # the context and its first blocks
+    before = torch.cuda.mem_get_info()[0]
+    s = b200.DeviceSystem(n, 0.01, precision="fp64")
+    taken = before - torch.cuda.mem_get_info()[0]
+    assert s.n == n and taken <= 80 * n + (8 << 20)
