@@ -99,6 +99,12 @@ const char *ob_version(void);
 const char *ob_last_error(void);
 int ob_device_count(int *count);
 
+/* Gives the device memory that the library keeps from destroyed objects for
+ * the next ones (at most 256 MB in the process) back to the device, for other
+ * allocators of the same process. The library does so by itself when an
+ * allocation of its own fails. No reference counterpart. */
+int ob_release_kept_memory(void);
+
 /* ------------------------------------------------------------------------ */
 /* Solver: the ForceSolver drop-in                                           */
 /* ------------------------------------------------------------------------ */

@@ -283,6 +283,12 @@ def device_count() -> int:
     return n.value
 
 
+def release_kept_memory() -> None:
+    """Gives the device memory kept from destroyed objects (at most 256 MB) back
+    to the device, for other allocators of this process."""
+    _check(load_library().ob_release_kept_memory())
+
+
 def _f64(a) -> np.ndarray:
     return np.ascontiguousarray(a, dtype=np.float64)
 

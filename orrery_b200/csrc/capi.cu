@@ -723,6 +723,10 @@ int ob_device_count(int *count) {
     });
 }
 
+int ob_release_kept_memory(void) {
+    return guarded([&] { ob::release_kept_blocks(); });
+}
+
 int ob_solver_create(const ob_solver_params *params, ob_solver **out) {
     return guarded([&] {
         require(out != nullptr && params != nullptr, "NULL argument");

@@ -107,6 +107,8 @@ void *take_device_block(size_t bytes, size_t &got, int &device) {
     return p;
 }
 
+void release_kept_blocks() { give_back(-1); }
+
 void keep_device_block(void *ptr, size_t bytes, int device) noexcept {
     if (bytes > kLargestKept) {
         cudaFree(ptr);

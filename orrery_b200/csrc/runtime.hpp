@@ -64,6 +64,8 @@ void *take_device_block(size_t bytes, size_t &got, int &device);
 // Keeps a block for the next object (bounded; else frees it). Nothing enqueued
 // on the device may still use it.
 void keep_device_block(void *ptr, size_t bytes, int device) noexcept;
+// Frees every kept block.
+void release_kept_blocks();
 
 // Owning device allocation that grows on demand and never shrinks, the
 // capacity policy of the reference's CUDA solvers

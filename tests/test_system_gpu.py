@@ -449,3 +449,18 @@ def test_a_large_block_takes_what_it_holds(b200):
     s = b200.DeviceSystem(n, 0.01, precision="fp64")
     taken = before - torch.cuda.mem_get_info()[0]
     assert s.n == n and taken <= 80 * n + (8 << 20)
+
+
+def test_kept_blocks_go_back_to_the_device_when_asked(b200):
+    torch = pytest.importorskip("torch")
+    from orrery_b200 import initial_conditions as ic
+    n = 400000  # 22 MB of staging
+    d = ic.plummer_sphere(n, seed=1)
+    b200.release_kept_memory()
+    b200.B200TreeSolver(0.02, 0.9, 32, False).evaluate((d["x"], d["y"], d["z"]), d["m"])
+    held = torch.cuda.mem_get_info()[0]
+    b200.release_kept_memory()
+    assert torch.cuda.mem_get_info()[0] - held >= 22 << 20
+    a = b200.B200DirectSolver(0.01, "fp64").evaluate(([0.0, 1.0], [0.0, 0.0], [0.0, 0.0]),
+                                                     [1.0, 1.0])
+    assert a[0, 0] > 0.9
