@@ -545,6 +545,14 @@ int ob_probe_fp64(double *dfma_lane_per_s);
  * look-back wait of the Morton ordering; no reference counterpart. */
 int ob_test_lookback_timeout(uint64_t n, uint32_t poll_limit, int skip_first_tile);
 
+/* In the next evaluation of the tree solver `solver` one CTA stays silent, and
+ * the build's waits end after `poll_limit` polls: stage 1, it does not arrive at
+ * the ordering's first barrier; 2, it does not publish the first sort pass's
+ * first tile; 3, it does not arrive at the layout's first barrier. An evaluation
+ * of more than 2,048 particles then reports OB_ERROR_TIMEOUT, and the one after
+ * it is as any other. No reference counterpart. */
+int ob_test_tree_timeout(ob_solver *solver, uint32_t stage, uint32_t poll_limit);
+
 /* Bounds the FP32 tree walk's traversal stack of `solver` to `cap` (at most
  * 256) entries (0 restores the full stack) from its next evaluation on. A group
  * of targets whose stack fills discards its partial sums and finishes with the

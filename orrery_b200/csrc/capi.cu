@@ -802,6 +802,18 @@ int ob_test_set_walk_stack_cap(ob_solver *solver, uint32_t cap) {
     });
 }
 
+int ob_test_tree_timeout(ob_solver *solver, uint32_t stage, uint32_t poll_limit) {
+    return guarded([&] {
+        require(solver != nullptr, "solver is NULL");
+        require(stage >= 1 && stage <= 3, "the build has three stages that can stay silent");
+        require(poll_limit > 0, "the poll limit must be positive");
+        if (solver->impl->params().kind != OB_SOLVER_TREE) {
+            throw ob::Error(OB_ERROR_UNSUPPORTED, "only a tree solver builds a tree");
+        }
+        solver->impl->tree().arm_timeout(static_cast<ob::SilentStage>(stage), poll_limit);
+    });
+}
+
 int ob_tree_stats(ob_solver *solver, uint64_t *nodes, uint64_t *leaves, uint32_t *depth) {
     return guarded([&] {
         require(solver != nullptr, "solver is NULL");

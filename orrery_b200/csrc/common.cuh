@@ -80,10 +80,11 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t *bar, uint32_t parity
 
 // A barrier of all CTAs of a cooperative launch (every CTA is resident): the
 // `count`-th barrier of the launch on `word`, which starts at zero. What any
-// CTA wrote before it is visible to loads from L2 (__ldcg) after it. Polls are
-// bounded: false (and kStatusTimeout) when the others never arrive, in which
-// case the caller returns.
-__device__ __forceinline__ bool grid_barrier(unsigned *word, unsigned count, unsigned *status) {
+// CTA wrote before it is visible to loads from L2 (__ldcg) after it. At most
+// `poll_limit` polls: false (and kStatusTimeout) when the others have not arrived
+// by then, in which case the caller returns.
+__device__ __forceinline__ bool grid_barrier(unsigned *word, unsigned count, unsigned *status,
+                                             uint32_t poll_limit) {
     __syncthreads();
     bool ok = true;
     if (threadIdx.x == 0) {
@@ -91,7 +92,7 @@ __device__ __forceinline__ bool grid_barrier(unsigned *word, unsigned count, uns
         atomicAdd(word, 1u);
         const unsigned target = count * gridDim.x;
         ok = false;
-        for (uint32_t poll = 0; poll < kSpinLimit && !ok; ++poll) {
+        for (uint32_t poll = 0; poll < poll_limit && !ok; ++poll) {
             unsigned seen;
             asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(word) : "memory");
             ok = seen >= target;

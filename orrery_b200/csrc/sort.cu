@@ -449,6 +449,8 @@ struct OrderArgs {
     TreeMeta *meta;
     unsigned *barrier;
     unsigned *status;
+    SilentStage silent;
+    uint32_t poll_limit;
 };
 
 struct OrderSpace {
@@ -461,6 +463,8 @@ struct OrderSpace {
     };
 };
 
+// TEST: a CTA stays silent at a.silent, and waits end after a.poll_limit polls.
+template <bool TEST>
 __global__ void __launch_bounds__(kSortThreads, 4) order_kernel(const OrderArgs a) {
     extern __shared__ __align__(16) unsigned char smem[];
     OrderSpace &space = *reinterpret_cast<OrderSpace *>(smem);
@@ -469,6 +473,18 @@ __global__ void __launch_bounds__(kSortThreads, 4) order_kernel(const OrderArgs 
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
     const uint32_t first = blockIdx.x * kSortThreads + tid, stride = gridDim.x * kSortThreads;
     unsigned barriers = 0;
+    const uint32_t poll_limit = TEST ? a.poll_limit : kLookbackPollLimit;
+    if (TEST && a.silent == SilentStage::ordering_barrier && blockIdx.x == 0 && gridDim.x > 1) {
+        return;
+    }
+    // All CTAs' barrier; false when this CTA is to return, the ordering abandoned.
+    auto meet = [&] {
+        const bool met = grid_barrier(a.barrier, ++barriers, a.status, poll_limit);
+        if (!met && tid == 0) {
+            atomicExch(&a.meta->node_count, 0u);
+        }
+        return met;
+    };
 
     // Nothing reads these words before the first barrier.
     for (size_t k = first; k < static_cast<size_t>(kRadixPasses) * kRadix; k += stride) {
@@ -494,7 +510,7 @@ __global__ void __launch_bounds__(kSortThreads, 4) order_kernel(const OrderArgs 
     if (tid < 6) {
         a.partials[blockIdx.x * 6 + tid] = mine;
     }
-    if (!grid_barrier(a.barrier, ++barriers, a.status)) {
+    if (!meet()) {
         return;
     }
 #pragma unroll
@@ -517,6 +533,7 @@ __global__ void __launch_bounds__(kSortThreads, 4) order_kernel(const OrderArgs 
     __syncthreads();
     if (tid == 0) {
         cube = TreeMeta{};
+        cube.node_count = kNodesUnset;
         write_cube(ext, a.n, &cube);
         if (blockIdx.x == 0) {
             *a.meta = cube; // the other scalars start at zero
@@ -526,10 +543,13 @@ __global__ void __launch_bounds__(kSortThreads, 4) order_kernel(const OrderArgs 
     __syncthreads();
     encode_particles(a.x, a.y, a.z, a.n, cube, space.encode.table, space.encode.local, a.keys[0],
                      a.perm[0], a.hist);
-    if (!grid_barrier(a.barrier, ++barriers, a.status)) {
+    if (!meet()) {
         return;
     }
 
+    if (TEST && a.silent == SilentStage::ordering_lookback && blockIdx.x == 0 && gridDim.x > 1) {
+        return;
+    }
     for (int pass = 0; pass < kRadixPasses; ++pass) {
         const bool odd = (pass & 1) != 0;
         const unsigned long long *keys_in = odd ? a.keys[1] : a.keys[0];
@@ -565,12 +585,15 @@ __global__ void __launch_bounds__(kSortThreads, 4) order_kernel(const OrderArgs 
                 if (!sort_one_tile(space.sort, tile, keys_in, perm_in, keys_out, perm_out, a.n,
                                    static_cast<uint32_t>(kRadixBits * pass), offset,
                                    a.lookback + static_cast<size_t>(pass) * a.tiles * kRadix,
-                                   a.status, kLookbackPollLimit)) {
-                    return; // the status word tells; the other CTAs' waits run out too
+                                   a.status, poll_limit)) {
+                    if (tid == 0) {
+                        atomicExch(&a.meta->node_count, 0u);
+                    }
+                    return; // the other CTAs' waits run out too
                 }
             }
         }
-        if (!grid_barrier(a.barrier, ++barriers, a.status)) {
+        if (!meet()) {
             return;
         }
     }
@@ -676,14 +699,17 @@ cudaError_t launch_order(const double *x, const double *y, const double *z, cons
                          uint32_t n, unsigned long long *const *keys, uint32_t *const *perm,
                          uint32_t *hist, uint32_t *lookback, double *partials, double *sorted,
                          uint32_t *zeroed, size_t zeroed_words, TreeMeta *meta,
-                         unsigned *barrier, unsigned *status, cudaStream_t stream) {
-    static std::atomic<uint64_t> configured{0};
-    static std::atomic<int> resident{0};
-    const void *kernel = reinterpret_cast<const void *>(order_kernel);
+                         unsigned *barrier, unsigned *status, cudaStream_t stream,
+                         SilentStage silent, uint32_t poll_limit) {
+    static std::atomic<uint64_t> configured[2];
+    static std::atomic<int> resident[2];
+    const bool test = silent != SilentStage::none;
+    const void *kernel = test ? reinterpret_cast<const void *>(order_kernel<true>)
+                              : reinterpret_cast<const void *>(order_kernel<false>);
     const uint32_t tiles = sort_tiles(n);
     uint32_t grid = 0;
     const cudaError_t err =
-        cooperative_grid(kernel, kSortThreads, sizeof(OrderSpace), configured, resident,
+        cooperative_grid(kernel, kSortThreads, sizeof(OrderSpace), configured[test], resident[test],
                          std::min(std::max(tiles, ceil_div(n, 1024u)), kMaxCooperativeBlocks),
                          grid);
     if (err != cudaSuccess) {
@@ -691,7 +717,7 @@ cudaError_t launch_order(const double *x, const double *y, const double *z, cons
     }
     OrderArgs a{x,        y,      z,      m,            n,    tiles,   {keys[0], keys[1]},
                 {perm[0], perm[1]}, hist,   lookback,     partials, sorted, zeroed,
-                zeroed_words,       meta,   barrier,      status};
+                zeroed_words,       meta,   barrier,      status,   silent, poll_limit};
     void *args[] = {&a};
     return cudaLaunchCooperativeKernel(kernel, dim3(grid), dim3(kSortThreads), args,
                                        sizeof(OrderSpace), stream);

@@ -26,6 +26,7 @@
 #include <algorithm>
 #include <atomic>
 #include <cmath>
+#include <utility>
 #include <vector>
 
 #include "common.cuh"
@@ -188,12 +189,30 @@ __device__ void node_run(const unsigned long long *codes, uint32_t n, uint32_t c
 // Node counts, their prefix sums and the node records in one cooperative
 // launch, with two grid barriers. Each CTA owns a contiguous share of the
 // particles; the prefix of a share is the sum of the totals before it.
+// TEST: CTA 0 stays silent at SilentStage::layout_barrier, and waits end after
+// `test_polls` polls.
+template <bool TEST>
 __global__ void __launch_bounds__(kThreads, 4)
     layout_kernel(const unsigned long long *__restrict__ codes, uint32_t n, uint32_t cap,
                   uint32_t *offsets, uint32_t *totals, uint32_t capacity, DeviceNode *nodes,
-                  uint32_t *child_mask, uint32_t *child_slots, TreeMeta *meta, unsigned *barrier,
-                  unsigned *status) {
+                  uint32_t *child_mask, uint32_t *child_slots, uint32_t *perm, TreeMeta *meta,
+                  unsigned *barrier, unsigned *status, SilentStage silent, uint32_t test_polls) {
     __shared__ uint32_t sums[kThreads / 32];
+    if (TEST && silent == SilentStage::layout_barrier && blockIdx.x == 0 && gridDim.x > 1) {
+        return;
+    }
+    // The codes of an abandoned ordering are not sorted: they are counted (every
+    // index up to the first barrier stays within the n codes, whatever they hold)
+    // but nothing is laid out, and the permutation, which the walks write
+    // through, becomes one. The load is on its way while the counts are formed.
+    const bool abandoned = __ldcg(&meta->node_count) == 0u;
+    auto meet = [&](unsigned count) {
+        const bool met = grid_barrier(barrier, count, status, TEST ? test_polls : kSpinLimit);
+        if (!met && threadIdx.x == 0) {
+            atomicExch(&meta->node_count, 0u);
+        }
+        return met;
+    };
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
     const uint32_t share = (n + gridDim.x - 1u) / gridDim.x;
     const uint32_t share_begin = min(static_cast<uint64_t>(blockIdx.x) * share,
@@ -236,7 +255,15 @@ __global__ void __launch_bounds__(kThreads, 4)
     if (tid == 0) {
         totals[blockIdx.x] = carry;
     }
-    if (!grid_barrier(barrier, 1u, status)) {
+    auto any_permutation = [&] {
+        for (uint32_t i = share_begin + tid; i < share_end; i += kThreads) {
+            perm[i] = i;
+        }
+    };
+    if (!meet(1u)) {
+        if (__syncthreads_or(abandoned ? 1 : 0) != 0) {
+            any_permutation();
+        }
         return;
     }
     // The nodes before this share, and all of them.
@@ -257,7 +284,10 @@ __global__ void __launch_bounds__(kThreads, 4)
         atomicAdd(&folded[0], before);
         atomicAdd(&folded[1], total);
     }
-    __syncthreads();
+    if (__syncthreads_or(abandoned ? 1 : 0) != 0) {
+        any_permutation();
+        return;
+    }
     before = folded[0];
     total = folded[1];
     for (uint32_t b = share_begin + tid; b < share_end; b += kThreads) {
@@ -266,11 +296,11 @@ __global__ void __launch_bounds__(kThreads, 4)
     if (blockIdx.x == 0 && tid == 0) {
         offsets[n] = total;
     }
-    if (!grid_barrier(barrier, 2u, status)) {
+    if (!meet(2u)) {
         return;
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) {
-        meta->node_count = total <= capacity ? total : 0u;
+        atomicCAS(&meta->node_count, kNodesUnset, total <= capacity ? total : 0u);
         meta->required = total;
         if (total > capacity) {
             atomicOr(status, kStatusOverflow);
@@ -612,20 +642,23 @@ uint32_t grid_for(uint32_t n) { return std::max(1u, std::min(ceil_div(n, kThread
 cudaError_t launch_layout(const unsigned long long *codes, uint32_t n, uint32_t leaf_cap,
                           uint32_t *offsets, uint32_t *totals, uint32_t node_capacity,
                           DeviceNode *nodes, uint32_t *child_mask, uint32_t *child_slots,
-                          TreeMeta *meta, unsigned *barrier, unsigned *status,
-                          cudaStream_t stream) {
-    static std::atomic<uint64_t> configured{0};
-    static std::atomic<int> resident{0};
-    const void *kernel = reinterpret_cast<const void *>(layout_kernel);
+                          uint32_t *perm, TreeMeta *meta, unsigned *barrier, unsigned *status,
+                          cudaStream_t stream, SilentStage silent, uint32_t poll_limit) {
+    static std::atomic<uint64_t> configured[2];
+    static std::atomic<int> resident[2];
+    const bool test = silent != SilentStage::none;
+    const void *kernel = test ? reinterpret_cast<const void *>(layout_kernel<true>)
+                              : reinterpret_cast<const void *>(layout_kernel<false>);
     uint32_t grid = 0;
-    const cudaError_t err = cooperative_grid(kernel, kThreads, 0, configured, resident,
+    const cudaError_t err = cooperative_grid(kernel, kThreads, 0, configured[test], resident[test],
                                              std::min(ceil_div(n, kThreads), kMaxCooperativeBlocks),
                                              grid);
     if (err != cudaSuccess) {
         return err;
     }
-    void *args[] = {&codes,        &n,     &leaf_cap,   &offsets,     &totals, &node_capacity,
-                    &nodes,        &child_mask, &child_slots, &meta,  &barrier, &status};
+    void *args[] = {&codes,      &n,           &leaf_cap, &offsets, &totals,
+                    &node_capacity, &nodes,    &child_mask, &child_slots, &perm,
+                    &meta,       &barrier,     &status,   &silent,  &poll_limit};
     return cudaLaunchCooperativeKernel(kernel, dim3(grid), dim3(kThreads), args, 0, stream);
 }
 
@@ -649,9 +682,6 @@ cudaError_t launch_moments(const double *sorted, const unsigned long long *codes
 // ---------------------------------------------------------------------------
 
 TreePipeline::TreePipeline(const ob_solver_params &params) : params_(params) {
-    int device = 0;
-    check(cudaGetDevice(&device), "cudaGetDevice");
-    check(cudaDeviceGetAttribute(&sm_count_, cudaDevAttrMultiProcessorCount, device), "SMs");
     meta_.reserve(1);
     check(cudaMemset(meta_.data(), 0, sizeof(TreeMeta)), "clearing tree scalars");
     counters_.reserve(2);
@@ -742,6 +772,8 @@ void TreePipeline::evaluate(uint32_t n, const double *x, const double *y, const 
     uint32_t *arrived = child_mask + node_capacity_;
     check(cudaMemsetAsync(barriers, 0, sizeof(unsigned) * kBarrierWords, stream),
           "clearing the barriers");
+    const SilentStage silent = std::exchange(silent_, SilentStage::none);
+    const uint32_t polls = std::exchange(poll_limit_, 0u);
 
     // Ordering: cube, codes, radix sort, gather; codes and permutation end in
     // buffer 0.
@@ -749,7 +781,7 @@ void TreePipeline::evaluate(uint32_t n, const double *x, const double *y, const 
     uint32_t *perms[2] = {perm_[0].data(), perm_[1].data()};
     check(launch_order(x, y, z, m, n, keys, perms, hist, lookback, reduce_.data(),
                        sorted_.data(), child_mask, 2ull * node_capacity_, meta_.data(), barriers,
-                       status, stream),
+                       status, stream, silent, polls),
           "ordering");
     const unsigned long long *codes = keys_[0].data();
     const uint32_t *perm = perm_[0].data();
@@ -763,8 +795,8 @@ void TreePipeline::evaluate(uint32_t n, const double *x, const double *y, const 
     const WalkNodes walk{records, records + node_capacity_, records + 2ull * node_capacity_,
                          records + 3ull * node_capacity_, walk_index_.data()};
     check(launch_layout(codes, n, cap, offsets, scan_partials_.data(), node_capacity_,
-                        nodes_.data(), child_mask, child_slots, meta_.data(), barriers + 1,
-                        status, stream),
+                        nodes_.data(), child_mask, child_slots, perms[0], meta_.data(), barriers + 1,
+                        status, stream, silent, polls),
           "node layout");
     check(launch_moments(sorted_.data(), codes, n, nodes_.data(),
                          params_.quadrupole ? quads_.data() : nullptr, walk, child_mask,

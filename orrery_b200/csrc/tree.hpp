@@ -58,12 +58,17 @@ struct DeviceQuadrupole {
     double xx, xy, xz, yy, yz, zz;
 };
 
+// The node count from the ordering to the layout, which replaces it (and nothing
+// else) by the number of nodes. A CTA whose wait ran out sets it to 0, for good:
+// the kernels after it then find no nodes.
+constexpr uint32_t kNodesUnset = 0xffffffffu;
+
 // Scalars the pipeline keeps on the device between its kernels.
 struct TreeMeta {
     double origin[3];
     double size;
     double root_centre[3];
-    uint32_t node_count;
+    uint32_t node_count; // kNodesUnset until the layout has them all; 0 once abandoned
     uint32_t leaf_count;
     uint32_t depth;
     uint32_t required;  // nodes the layout needed (reported on overflow)
@@ -71,6 +76,14 @@ struct TreeMeta {
     uint32_t reserved;
     unsigned long long pairs;
     unsigned long long cells;
+};
+
+// Where a CTA stays silent in a test of the build's bounded waits.
+enum class SilentStage : uint32_t {
+    none,
+    ordering_barrier,  // does not arrive at the ordering's first barrier
+    ordering_lookback, // does not publish the first sort pass's first tile
+    layout_barrier     // does not arrive at the layout's first barrier
 };
 
 class TreePipeline {
@@ -110,6 +123,13 @@ public:
     // per-target union walk. For tests of that fallback.
     void set_walk_stack_cap(uint32_t cap) noexcept { walk_stack_cap_ = cap; }
 
+    // Tests of the build's bounded waits: in the next evaluation a CTA stays
+    // silent at `stage`, and every wait ends after `poll_limit` polls.
+    void arm_timeout(SilentStage stage, uint32_t poll_limit) noexcept {
+        silent_ = stage;
+        poll_limit_ = poll_limit;
+    }
+
     // The device scalars of the last evaluation (synchronous).
     TreeMeta meta();
 
@@ -128,7 +148,8 @@ private:
     uint64_t generation_ = 0;
     uint32_t last_n_ = 0;
     uint32_t walk_stack_cap_ = 0;
-    int sm_count_ = 148;
+    SilentStage silent_ = SilentStage::none;
+    uint32_t poll_limit_ = 0; // 0: the kernels' own limit
     DeviceArray<unsigned long long> keys_[2];    // Morton codes (double-buffered)
     DeviceArray<uint32_t> perm_[2];              // particle index payload
     DeviceArray<uint32_t> scratch_;              // barrier counts, digit histograms, look-back

@@ -72,13 +72,16 @@ cudaError_t cooperative_grid(const void *kernel, int threads, size_t smem,
 // = source_k[perm[0][i]] for x, y, z, m; *meta's other scalars and the
 // `zeroed_words` words at `zeroed` are zeroed on the way. `barrier` (one word)
 // is zero at the start; hist, lookback (of all passes) and `partials`
-// (order_partials_needed() doubles) are scratch.
+// (order_partials_needed() doubles) are scratch. A bounded wait that ran out sets
+// kStatusTimeout and leaves no nodes (kNodesUnset, tree.hpp). With a
+// `silent` stage (tests) the waits end after `poll_limit` polls.
 size_t order_partials_needed();
 cudaError_t launch_order(const double *x, const double *y, const double *z, const double *m,
                          uint32_t n, unsigned long long *const *keys, uint32_t *const *perm,
                          uint32_t *hist, uint32_t *lookback, double *partials, double *sorted,
                          uint32_t *zeroed, size_t zeroed_words, TreeMeta *meta,
-                         unsigned *barrier, unsigned *status, cudaStream_t stream);
+                         unsigned *barrier, unsigned *status, cudaStream_t stream,
+                         SilentStage silent = SilentStage::none, uint32_t poll_limit = 0);
 
 // ------------------------------------------------------------------ octree
 
@@ -87,12 +90,15 @@ cudaError_t launch_order(const double *x, const double *y, const double *z, cons
 // level, parent, octant), and each internal node's children by octant, marked
 // in child_mask (zeroed beforehand) and listed in its kMaxChildren child_slots.
 // `totals` holds kMaxCooperativeBlocks words; `barrier` is zero at the start.
+// After an abandoned ordering it lays out nothing and makes `perm` a permutation,
+// so that the walks read and write nothing out of range.
 constexpr uint32_t kMaxChildren = 8;
 cudaError_t launch_layout(const unsigned long long *codes, uint32_t n, uint32_t leaf_cap,
                           uint32_t *offsets, uint32_t *totals, uint32_t node_capacity,
                           DeviceNode *nodes, uint32_t *child_mask, uint32_t *child_slots,
-                          TreeMeta *meta, unsigned *barrier, unsigned *status,
-                          cudaStream_t stream);
+                          uint32_t *perm, TreeMeta *meta, unsigned *barrier, unsigned *status,
+                          cudaStream_t stream, SilentStage silent = SilentStage::none,
+                          uint32_t poll_limit = 0);
 
 // Moments bottom-up (mass, centre of mass, quadrupole, acceptance radius) and
 // the leaf-relative FP32 source positions the walk reads.

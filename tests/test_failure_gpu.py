@@ -52,6 +52,48 @@ def test_the_test_entry_checks_its_arguments(b200):
     assert fn((1 << 24) + 1, 10, 0) == b200.ERROR_INVALID_ARGUMENT
 
 
+@pytest.mark.parametrize("precision", ["fp32", "fp64"])
+@pytest.mark.parametrize("stage", [1, 2, 3])
+def test_a_silent_cta_of_the_tree_build_times_out_and_the_next_build_is_whole(b200, restatement,
+                                                                              stage, precision):
+    # One CTA does not arrive at a grid barrier of the ordering (1) or of the
+    # layout (3), or does not publish its tile of a sort pass (2). The others'
+    # waits run out and the kernels after them index nothing; the solver's
+    # first evaluation has no permutation yet that they could use by chance.
+    from orrery_b200 import initial_conditions as ic
+    lib = b200.load_library()
+    lib.ob_test_tree_timeout.argtypes = [C.c_void_p, C.c_uint32, C.c_uint32]
+    d = ic.plummer_sphere(20_011, seed=stage)
+    x, y, z, m = d["x"], d["y"], d["z"], d["m"]
+    solver = b200.B200TreeSolver(0.02, 0.6, 16, True, precision)
+    for _ in range(2):
+        assert lib.ob_test_tree_timeout(solver._handle, stage, 5000) == b200.OK
+        with pytest.raises(b200.OrreryError) as err:
+            solver.evaluate((x, y, z), m)
+        assert err.value.code == b200.ERROR_TIMEOUT
+        solver.reset_interaction_count()
+        a = solver.evaluate((x, y, z), m)
+        c = solver.interaction_count()
+        fresh = b200.B200TreeSolver(0.02, 0.6, 16, True, precision)
+        assert np.array_equal(a, fresh.evaluate((x, y, z), m))
+        a_ref, counts = restatement.barnes_hut(x, y, z, m, 0.02, 0.6, 16, True)
+        assert (c.particle_particle, c.particle_cell) == (counts.particle_particle,
+                                                          counts.particle_cell)
+        if precision == "fp64":
+            assert np.array_equal(a, a_ref)
+
+
+def test_the_tree_timeout_entry_checks_its_arguments(b200):
+    lib = b200.load_library()
+    lib.ob_test_tree_timeout.argtypes = [C.c_void_p, C.c_uint32, C.c_uint32]
+    tree = b200.B200TreeSolver(0.01, 0.5, 32, True)
+    assert lib.ob_test_tree_timeout(tree._handle, 0, 10) == b200.ERROR_INVALID_ARGUMENT
+    assert lib.ob_test_tree_timeout(tree._handle, 4, 10) == b200.ERROR_INVALID_ARGUMENT
+    assert lib.ob_test_tree_timeout(tree._handle, 1, 0) == b200.ERROR_INVALID_ARGUMENT
+    direct = b200.B200DirectSolver(0.01)
+    assert lib.ob_test_tree_timeout(direct._handle, 1, 10) == b200.ERROR_UNSUPPORTED
+
+
 @pytest.mark.parametrize("cap", [2, 24, 64])
 def test_a_full_traversal_stack_falls_back_to_the_union_walk(b200, restatement, cap):
     # A stack capped at a few entries fills in (almost) every warp, which then
