@@ -378,9 +378,8 @@ bool Solver::grew_after_overflow(cudaStream_t stream) {
     if (status & kStatusTimeout) {
         throw Error(OB_ERROR_TIMEOUT, "a device-side wait ran out of its bound");
     }
-    if (status & kStatusInvalid) {
-        throw Error(OB_ERROR_CUDA, "a kernel met an index its data structure cannot hold");
-    }
+    // A tree that outgrew its nodes has none, so the FP32 walk has met an index
+    // past the last one: looked at first.
     if ((status & kStatusOverflow) && tree_) {
         const uint32_t required = tree_->meta().required;
         tree_->grow_nodes(required + required / 4 + 1024);
@@ -388,6 +387,9 @@ bool Solver::grew_after_overflow(cudaStream_t stream) {
     }
     if (status & kStatusOverflow) {
         throw Error(OB_ERROR_CAPACITY, "a device-side buffer bound was exceeded");
+    }
+    if (status & kStatusInvalid) {
+        throw Error(OB_ERROR_CUDA, "a kernel met an index its data structure cannot hold");
     }
     return false;
 }
@@ -397,11 +399,11 @@ void Solver::check_status(cudaStream_t stream) {
     if (status & kStatusTimeout) {
         throw Error(OB_ERROR_TIMEOUT, "a device-side wait ran out of its bound");
     }
+    if (status & kStatusOverflow) { // and what follows from it (grew_after_overflow)
+        throw Error(OB_ERROR_CAPACITY, "a device-side buffer bound was exceeded");
+    }
     if (status & kStatusInvalid) {
         throw Error(OB_ERROR_CUDA, "a kernel met an index its data structure cannot hold");
-    }
-    if (status & kStatusOverflow) {
-        throw Error(OB_ERROR_CAPACITY, "a device-side buffer bound was exceeded");
     }
 }
 

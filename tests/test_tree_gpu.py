@@ -92,6 +92,28 @@ def test_ragged_sizes_and_parameters_against_oracle(b200, restatement, n, leaf, 
         assert a.tolist() == [[0.0, 0.0, 0.0]]
 
 
+@pytest.mark.parametrize("precision", ["fp32", "fp64"])
+def test_a_tree_that_outgrows_its_nodes_is_built_again(b200, restatement, precision):
+    # Tight clusters of one particle more than a leaf holds: a chain of cells
+    # each, beyond the nodes reserved for the particle count.
+    rng = np.random.default_rng(4)
+    centres = rng.uniform(-1.0, 1.0, (2000, 3))
+    p = np.repeat(centres, 5, axis=0) + 1e-6 * rng.normal(size=(10000, 3))
+    x, y, z = (np.ascontiguousarray(p[:, k]) for k in range(3))
+    m = rng.uniform(0.5, 1.5, len(x))
+    a_ref, counts = restatement.barnes_hut(x, y, z, m, 0.01, 0.5, 4, True)
+    s = b200.B200TreeSolver(0.01, 0.5, 4, True, precision)
+    a = s.evaluate((x, y, z), m)
+    c = s.interaction_count()
+    assert (c.particle_particle, c.particle_cell) == (counts.particle_particle,
+                                                      counts.particle_cell)
+    assert s.tree_stats()[0] > 8 * len(x) // 4 + len(x) // 2 + 1024  # what was reserved
+    if precision == "fp64":
+        assert np.array_equal(a, a_ref)
+    else:
+        assert relative_errors(a, a_ref).max() < TREE_WORST
+
+
 # 2,048 keys make a sort tile; 1,212,417 make one more than the ordering's CTAs.
 @pytest.mark.parametrize("n", [2047, 2048, 2049, 151553, 1212417])
 def test_ordering_and_layout_at_the_edges_of_tiles(b200, restatement, n):
