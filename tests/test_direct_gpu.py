@@ -83,9 +83,9 @@ _FACTORS = {-5: [3, 7, 140627, 173331457829, 158494480927183],
 
 
 def _hard_arguments():
-    """The x whose square root, or the reciprocal of whose square root, lies so
-    near a midpoint of two doubles that a result good to 2^-103 before its last
-    rounding could round wrongly."""
+    """Every x whose square root, or the reciprocal of whose rounded square root,
+    lies so near a midpoint of two doubles that a result good to 2^-103 before its
+    last rounding could round wrongly (at a few exponents each)."""
     found = []
     # Roots: M^2 - j = x 2^k with M an odd 54-bit integer (a midpoint) and
     # |j| <= 2 M^2 2^-103 < 64; x in [1, 2) and [2, 4) stand for every x.
@@ -98,7 +98,8 @@ def _hard_arguments():
                         found += [np.ldexp(float(square >> k), k - 54 - 52 + 2 * e)
                                   for e in (-420, -120, 0, 17, 350)]
     # Reciprocals: s M = 2^106 - j with s a 53-bit integer, M a 54-bit odd one
-    # and |j| <= 2^106 2^-103.8 < 5; x = s^2, whose rounded root is s again.
+    # and |j| <= 2^106 2^-103.8 < 5; all x whose rounded root is s: s^2 rounded
+    # and its neighbours.
     for j, primes in _FACTORS.items():
         n = (1 << 106) - j
         divisors = {1}
@@ -107,8 +108,15 @@ def _hard_arguments():
         assert max(divisors) == n
         for s in divisors:
             if 1 << 52 <= s < 1 << 53 and (n // s) % 2 == 1:
-                found += [float(np.ldexp(float(s), e - 52)) ** 2 for e in (-440, -53, 0, 1, 300)]
+                for e in (-440, -53, 0, 1, 300):
+                    root = float(np.ldexp(float(s), e - 52))
+                    for direction in (0.0, np.inf):
+                        x = root ** 2
+                        while np.sqrt(x) == root:
+                            found.append(float(x))
+                            x = np.nextafter(x, direction)
     edges = [np.nextafter(4.0 ** k, 0) for k in (-200, 0, 1, 2, 300)]
+    edges += [np.nextafter(x, 0) for x in edges]  # both round to the root 2 - 2^-52
     return found + edges + [2.0 ** k for k in range(-1074, 1024, 53)]
 
 
