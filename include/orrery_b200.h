@@ -176,8 +176,9 @@ int ob_morton_order_noalloc(uint64_t n, const double *x, const double *y, const 
                             void *stream);
 
 /* Tile shape of the direct kernels: threads per CTA, targets per thread, the
- * number of CTAs (parts) that split the sources of a target tile, and the number of thread groups of a CTA that split each
- * staged tile's sources (each group serves the CTA's targets; 0 reads as 1).
+ * number of CTAs (parts) that split the sources of a target tile, and the
+ * number of thread groups of a CTA that split each staged tile's sources (each
+ * group serves the CTA's targets; 0 reads as 1).
  * A CTA holds threads * targets_per_thread / groups targets. No reference
  * counterpart: the reference picks one block size
  * (src/solvers/cuda_direct_solver.cpp:46-63). */
@@ -195,8 +196,9 @@ int ob_direct_shapes(int32_t precision, ob_direct_shape *out, int32_t capacity, 
 /* Fixes the shape a direct solver uses for n particles. */
 int ob_solver_set_direct_shape(ob_solver *solver, uint64_t n, const ob_direct_shape *shape);
 
-/* Times every implemented shape on the device for n synthetic particles and
- * keeps the fastest for n; returns it and its time per evaluation. */
+/* Times every implemented shape (the one taken without tuning among them) on the
+ * device for n synthetic particles and keeps the fastest for n; returns it and
+ * its time per evaluation. */
 int ob_solver_autotune(ob_solver *solver, uint64_t n, ob_direct_shape *chosen, double *best_ms);
 
 /* ------------------------------------------------------------------------ */

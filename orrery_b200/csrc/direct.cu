@@ -28,6 +28,7 @@
 //     parts are added in order, so the result does not depend on scheduling.
 #include <algorithm>
 #include <cooperative_groups.h>
+#include <iterator>
 
 #include "common.cuh"
 #include "f64_math.cuh"
@@ -809,20 +810,24 @@ uint32_t targets_per_cta(const DirectConfig &c) {
 
 } // namespace
 
+// Sums of all parts, were they to meet in memory.
+static size_t parts_doubles(uint32_t n, const DirectConfig &c) {
+    const uint32_t bt = targets_per_cta(c);
+    return 3ull * bt * ceil_div(n, bt) * static_cast<size_t>(c.split);
+}
+
 bool direct_uses_cluster(uint32_t n, const DirectConfig &c) {
-    // The grid fits the SMs at two CTAs each, and the parts a portable cluster.
+    // The parts fit a portable cluster, and either the grid fits the SMs at two
+    // CTAs each or the sums would take more memory than parts may.
     const bool portable = c.split == 1 || c.split == 2 || c.split == 4 || c.split == 8;
-    return portable && (c.split == 1 || static_cast<uint64_t>(ceil_div(n, targets_per_cta(c))) *
-                                                static_cast<uint64_t>(c.split) <=
-                                            2u * 148u);
+    const uint64_t ctas = static_cast<uint64_t>(ceil_div(n, targets_per_cta(c))) *
+                          static_cast<uint64_t>(c.split);
+    return portable && (c.split == 1 || ctas <= 2u * 148u ||
+                        parts_doubles(n, c) * sizeof(double) > kDirectPartsBytes);
 }
 
 size_t direct_partial_doubles(uint32_t n, const DirectConfig &c) {
-    if (direct_uses_cluster(n, c)) {
-        return 0;
-    }
-    const uint32_t bt = targets_per_cta(c);
-    return 3ull * bt * ceil_div(n, bt) * static_cast<size_t>(c.split);
+    return direct_uses_cluster(n, c) ? 0 : parts_doubles(n, c);
 }
 
 size_t direct_arrival_words(uint32_t n, const DirectConfig &c) {
@@ -910,6 +915,24 @@ cudaError_t launch_direct_f64(const double *x, const double *y, const double *z,
     return cudaGetLastError();
 }
 
+// The shapes and parts among which direct_default_config chooses.
+struct DefaultShape {
+    int targets, groups;
+    double per_pair; // cost per pair beside the cheapest one
+};
+struct DefaultShapes {
+    const DefaultShape *shapes;
+    int count;
+};
+constexpr int kDefaultThreads = 256;
+static const int kDefaultParts[] = {1, 2, 4, 8, 3, 5, 6, 10, 12, 16, 24, 32};
+
+static DefaultShapes default_shapes(bool split) {
+    static const DefaultShape fp32_shapes[] = {{4, 8, 1.0}, {2, 8, 1.01}};
+    static const DefaultShape split_shapes[] = {{4, 8, 1.0}, {4, 4, 0.985}, {2, 8, 1.06}};
+    return split ? DefaultShapes{split_shapes, 3} : DefaultShapes{fp32_shapes, 2};
+}
+
 int direct_candidates(bool split, DirectConfig *out, int capacity) {
     // (threads, targets per thread, source groups). 64-thread CTAs and source
     // groups give small systems (a few thousand particles) enough warps to
@@ -925,12 +948,24 @@ int direct_candidates(bool split, DirectConfig *out, int capacity) {
     const int shape_count = split ? 12 : 14;
     static const int splits[] = {1, 2, 4, 8};
     int count = 0;
+    auto add = [&](int threads, int targets, int parts, int groups) {
+        if (count < capacity) {
+            out[count] = DirectConfig{threads, targets, parts, groups};
+        }
+        ++count;
+    };
     for (int s = 0; s < shape_count; ++s) {
-        for (int k = 0; k < 4; ++k) {
-            if (count < capacity) {
-                out[count] = DirectConfig{shapes[s][0], shapes[s][1], splits[k], shapes[s][2]};
+        for (const int parts : splits) {
+            add(shapes[s][0], shapes[s][1], parts, shapes[s][2]);
+        }
+    }
+    // The other parts that the default rule takes, with the shapes that it takes.
+    const DefaultShapes rule = default_shapes(split);
+    for (int s = 0; s < rule.count; ++s) {
+        for (const int parts : kDefaultParts) {
+            if (std::find(std::begin(splits), std::end(splits), parts) == std::end(splits)) {
+                add(kDefaultThreads, rule.shapes[s].targets, parts, rule.shapes[s].groups);
             }
-            ++count;
         }
     }
     return count;
@@ -956,9 +991,6 @@ static double direct_cost(const DirectConfig &c, double per_pair, uint32_t n, ui
     return cost;
 }
 
-// Memory the parts' sums may take (a large system gains nothing from parts).
-constexpr size_t kPartsBytes = size_t{64} << 20;
-
 DirectConfig direct_default_config(uint32_t n, bool split, int sm_count) {
     // The cheapest of a few 256-thread shapes by the estimate above, whose
     // constants are fitted to sweeps from 1,000 to 262,144 particles on B200.
@@ -968,31 +1000,23 @@ DirectConfig direct_default_config(uint32_t n, bool split, int sm_count) {
     // 1,737; split sums of 10,007 and 65,536 178 us and 5.0 ms, now 127 us and
     // 4.2 ms.
     const uint32_t sms = static_cast<uint32_t>(sm_count > 0 ? sm_count : 148);
-    struct Shape {
-        int targets, groups;
-        double per_pair;
-    };
-    static const Shape fp32_shapes[] = {{4, 8, 1.0}, {2, 8, 1.01}};
-    static const Shape split_shapes[] = {{4, 8, 1.0}, {4, 4, 0.985}, {2, 8, 1.06}};
-    static const int parts_tried[] = {1, 2, 4, 8, 3, 5, 6, 10, 12, 16, 24, 32};
-    const Shape *shapes = split ? split_shapes : fp32_shapes;
-    const int shape_count = split ? 3 : 2;
+    const DefaultShapes rule = default_shapes(split);
     DirectConfig best;
     double best_cost = 0.0;
-    for (int k = 0; k < shape_count; ++k) {
-        for (const int parts : parts_tried) {
+    for (int k = 0; k < rule.count; ++k) {
+        for (const int parts : kDefaultParts) {
             if (parts > 1 && static_cast<uint32_t>(parts) > ceil_div(n, kDirectTile)) {
                 continue;
             }
             DirectConfig c;
-            c.threads = 256;
-            c.targets_per_thread = shapes[k].targets;
-            c.groups = shapes[k].groups;
+            c.threads = kDefaultThreads;
+            c.targets_per_thread = rule.shapes[k].targets;
+            c.groups = rule.shapes[k].groups;
             c.split = parts;
-            if (direct_partial_doubles(n, c) * sizeof(double) > kPartsBytes) {
-                continue;
+            if (parts_doubles(n, c) * sizeof(double) > kDirectPartsBytes) {
+                continue; // a large system gains nothing from parts
             }
-            const double cost = direct_cost(c, shapes[k].per_pair, n, sms);
+            const double cost = direct_cost(c, rule.shapes[k].per_pair, n, sms);
             if (best_cost == 0.0 || cost < best_cost) {
                 best = c;
                 best_cost = cost;

@@ -41,6 +41,8 @@ struct DirectParts {
     double *sums = nullptr;
     unsigned *arrived = nullptr;
 };
+// Device memory the parts' sums may take.
+constexpr size_t kDirectPartsBytes = size_t{64} << 20;
 bool direct_uses_cluster(uint32_t n, const DirectConfig &config);
 size_t direct_partial_doubles(uint32_t n, const DirectConfig &config);
 size_t direct_arrival_words(uint32_t n, const DirectConfig &config);

@@ -238,12 +238,21 @@ double Solver::autotune(uint32_t n, DirectConfig &chosen) {
     double *out = dev.data() + 4ull * n;
     for (int k = 0; k < count && k < 128; ++k) {
         const DirectConfig c = candidates[k];
-        if (static_cast<uint32_t>(c.split) > ceil_div(n, kDirectTile)) {
+        if (static_cast<uint32_t>(c.split) > ceil_div(n, kDirectTile) ||
+            direct_partial_doubles(n, c) * sizeof(double) > kDirectPartsBytes) {
             continue;
         }
         const uint32_t padded = direct_padded_count(n, c);
         hi_.reserve((split ? 2ull : 1ull) * padded);
-        const DirectParts parts = reserve_parts(n, c);
+        DirectParts parts;
+        try {
+            parts = reserve_parts(n, c);
+        } catch (const Error &e) {
+            if (e.code() != OB_ERROR_OUT_OF_MEMORY) {
+                throw;
+            }
+            continue; // no room for this one's sums
+        }
         if (split) {
             lo_.reserve(2ull * padded);
         }

@@ -321,3 +321,55 @@ def test_parts_are_added_in_order_wherever_they_meet(b200, restatement, precisio
         assert np.median(err) < SPLIT_MEDIAN and err.max() < 1e-5
     for _ in range(2):
         assert np.array_equal(s.evaluate((x, y, z), m), a)
+
+
+def _kernel_ms(s, n, xyz, m):
+    times = []
+    for _ in range(15):
+        s.evaluate(xyz, m)
+        times.append(s.timings()["traversal_ms"])
+    return np.median(times)
+
+
+@pytest.mark.parametrize("precision,n", [("split", 1500), ("split", 2500), ("fp32", 5003)])
+def test_tuning_never_picks_a_slower_shape_than_none(b200, precision, n):
+    # The default takes three and five parts here; the best shapes of 1, 2, 4 or 8
+    # parts were 37, 38 and 16 % slower. 8 %: the noise of these short kernels.
+    from orrery_b200 import initial_conditions as ic
+    d = ic.plummer_sphere(n, seed=n)
+    xyz, m = (d["x"], d["y"], d["z"]), d["m"]
+    untuned = _kernel_ms(b200.B200DirectSolver(0.05, precision), n, xyz, m)
+    s = b200.B200DirectSolver(0.05, precision)
+    shape, _ = s.autotune(n)
+    assert _kernel_ms(s, n, xyz, m) < 1.08 * untuned
+    # What tuning returns can be set by hand.
+    again = b200.B200DirectSolver(0.05, precision)
+    again.set_shape(n, shape)
+    assert np.array_equal(again.evaluate(xyz, m), s.evaluate(xyz, m))
+
+
+def test_parts_take_a_bounded_amount_of_memory(b200):
+    # Eight parts of a million targets would leave 192 MB of sums in memory; they
+    # meet in clusters instead.
+    torch = pytest.importorskip("torch")
+    n = 1 << 20
+    rng = torch.Generator(device="cuda")
+    rng.manual_seed(3)
+    x = torch.rand(3, n, generator=rng, device="cuda", dtype=torch.float64)
+    m = torch.full((n,), 1.0 / n, device="cuda", dtype=torch.float64)
+    out = torch.zeros(3, n, device="cuda", dtype=torch.float64)
+    s = b200.B200DirectSolver(0.05, "fp32")
+    s.set_shape(n, (256, 4, 8, 8))
+    torch.cuda.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    s.evaluate_device(n, x[0], x[1], x[2], m, out[0], out[1], out[2],
+                      torch.cuda.current_stream().cuda_stream)
+    torch.cuda.synchronize()
+    # 16 bytes of packed sources per particle, and what parts may take.
+    assert before - torch.cuda.mem_get_info()[0] < 16 * n + (64 << 20) + (8 << 20)
+    some = torch.arange(0, n, 4099, device="cuda")
+    for i in some.tolist()[:64]:
+        diff = x - x[:, i:i + 1]
+        w = m * ((diff * diff).sum(0) + 0.05 ** 2) ** -1.5
+        exact = (diff * w).sum(1)
+        assert float((out[:, i] - exact).norm() / exact.norm()) < FP32_WORST
