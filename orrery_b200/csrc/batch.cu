@@ -354,6 +354,7 @@ Batch::~Batch() {
         items_.keep();
         side_items_.keep();
         groups_.keep();
+        side_groups_.keep();
         partial_.keep();
         queue_.keep();
         status_.keep();
@@ -634,25 +635,35 @@ void Batch::refresh_members(const std::vector<uint32_t> &ids) {
     if (ids.empty()) {
         return;
     }
-    // Whole-system items (no partial slots) for just these members.
-    BatchConfig whole = config_;
-    whole.chunk_tiles = 0;
+    // The same items as in an evaluation of every member, so the same sums. They
+    // are some of those, so the partial slots suffice.
+    rebuild_if_needed();
     std::vector<BatchGroup> groups;
     uint32_t slots = 0;
-    const std::vector<BatchItem> items = make_items(whole, ids, groups, slots);
-    side_items_.reserve(items.size()); // the step graph never reads side_items_
+    const std::vector<BatchItem> items = make_items(config_, ids, groups, slots);
+    side_items_.reserve(items.size()); // the step graph reads neither of the two
+    side_groups_.reserve(std::max<size_t>(1, groups.size()));
     check(cudaMemcpyAsync(side_items_.data(), items.data(), sizeof(BatchItem) * items.size(),
                           cudaMemcpyHostToDevice, stream_),
           "uploading work items");
+    if (!groups.empty()) {
+        check(cudaMemcpyAsync(side_groups_.data(), groups.data(),
+                              sizeof(BatchGroup) * groups.size(), cudaMemcpyHostToDevice, stream_),
+              "uploading reduction groups");
+    }
     check(pack_sources(array(kX), array(kY), array(kZ), array(kM), high_, high_, hi_.data(),
                        lo_.data(), stream_),
           "packing sources");
     check(cudaMemsetAsync(queue_.data(), 0, sizeof(uint32_t), stream_), "resetting the queue");
     check(launch_batch_forces(hi_.data(), lo_.data(), eps2_.data(), side_items_.data(),
-                              static_cast<uint32_t>(items.size()), whole, array(kAx), array(kAy),
-                              array(kAz), partial_.data(), queue_.data(), status_.data(),
-                              sm_count_, stream_),
+                              static_cast<uint32_t>(items.size()), config_, array(kAx),
+                              array(kAy), array(kAz), partial_.data(), queue_.data(),
+                              status_.data(), sm_count_, stream_),
           "batched forces");
+    check(launch_batch_reduce(side_groups_.data(), static_cast<uint32_t>(groups.size()),
+                              partial_.data(), config_.targets_per_block(), array(kAx), array(kAy),
+                              array(kAz), stream_),
+          "reducing partial sums");
     check(cudaStreamSynchronize(stream_), "evaluating new members");
 }
 

@@ -177,7 +177,8 @@ private:
     DeviceArray<float4> lo_;
     DeviceArray<float> eps2_;
     DeviceArray<BatchItem> items_;
-    DeviceArray<BatchItem> side_items_;
+    DeviceArray<BatchItem> side_items_;  // of refresh_members
+    DeviceArray<BatchGroup> side_groups_;
     DeviceArray<BatchGroup> groups_;
     DeviceArray<double> partial_;
     DeviceArray<uint32_t> queue_;

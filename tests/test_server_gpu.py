@@ -68,6 +68,28 @@ def test_served_direct_job_tracks_the_precision_system(b200):
     assert np.max(np.abs(final["vy"] - st["vy"])) < 1e-8
 
 
+# Sizes with one, two and more chunks of sources: a joining member's first
+# evaluation and one of the whole batch sum alike.
+@pytest.mark.parametrize("n", [700, 1500, 3000, 9000])
+def test_served_direct_job_equals_the_batch(b200, n):
+    d = dict(_direct(n, 13))
+    # Masses over ten decades: a target's partial sums then differ enough in size
+    # for their order to show.
+    d["m"] = 10.0 ** np.random.default_rng(n).uniform(-10, 0, n)
+    server = _server(b200)
+    # A long step, so that the last bits of the first accelerations show.
+    ids = [server.submit(d, steps=2, dt=0.5, softening=0.01),
+           server.submit(_direct(2000, 14), steps=2, dt=0.5, softening=0.01)]
+    final = [server.wait(i, timeout=120) for i in ids][0][1]
+    server.close()
+    batch = b200.DeviceBatch([n], [0.01])
+    batch.set_state(0, d["x"], d["y"], d["z"], d["vx"], d["vy"], d["vz"], d["m"])
+    batch.refresh()
+    batch.step(0.5, 2, "yoshida4")
+    st = batch.state(0)
+    assert all(np.array_equal(final[k], st[k]) for k in KEYS)
+
+
 def test_served_tree_job_equals_the_device_system(b200):
     d = _tree(50000, 12)
     server = _server(b200)
