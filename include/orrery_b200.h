@@ -398,10 +398,14 @@ int ob_trajectory_close(ob_trajectory *trajectory);
  * replayed CUDA graph. */
 typedef struct ob_batch ob_batch;
 
+#define OB_BATCH_CHUNKS_BY_SIZE 0xffffffffu
+
 typedef struct ob_batch_shape {
     int32_t threads;
     int32_t targets_per_thread;
-    uint32_t chunk_tiles; /* 512-source tiles per work item; 0 = a whole system */
+    uint32_t chunk_tiles; /* 512-source tiles per work item; 0 = a whole system,
+                           * OB_BATCH_CHUNKS_BY_SIZE = by each system's own size
+                           * (a batch's default) */
     int32_t groups;       /* thread groups splitting each tile's sources; 0 reads as 1 */
 } ob_batch_shape;
 

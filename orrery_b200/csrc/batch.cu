@@ -784,7 +784,8 @@ void Batch::energy(uint32_t id, double *kinetic, double *potential) {
 }
 
 double Batch::autotune(BatchConfig &chosen) {
-    static const uint32_t chunks[] = {0, 16, 8, 4};
+    // Chunks by size, the default, among them.
+    static const uint32_t chunks[] = {kChunkBySize, 0, 16, 8, 4};
     cudaEvent_t start, stop;
     check(cudaEventCreate(&start), "event");
     check(cudaEventCreate(&stop), "event");

@@ -46,7 +46,7 @@ struct BatchGroup {
 // small systems (four of 256 to 4,096: a Yoshida step 197 us, whole systems per
 // item 308 us); eight tiles bound the end of the queue (one system of 16,384:
 // 1.04 ms, whole 1.99 ms) at 3 % more time than whole systems in a large batch.
-constexpr uint32_t kChunkBySize = 0xffffffffu;
+constexpr uint32_t kChunkBySize = OB_BATCH_CHUNKS_BY_SIZE;
 
 // Tile shape of the batched kernel.
 struct BatchConfig {

@@ -189,3 +189,40 @@ def test_invalid_batches_are_refused(b200):
         b200.DeviceBatch([100, 200], [0.01, 0.0])   # a zero softening
     with pytest.raises(b200.OrreryError):
         b200.DeviceBatch([100, 0], [0.01, 0.01])    # an empty system
+
+
+def test_tuning_times_the_default_s_chunks(b200):
+    # One system of 2,048: chunks by size take two tiles, a third less time than the
+    # fixed chunks that tuning tries (four tiles or more). 8 %: the noise.
+    import time
+
+    from orrery_b200 import initial_conditions as ic
+    n, by_size = 2048, 0xffffffff
+    d = ic.plummer_sphere(n, seed=n)
+
+    def batch(shape=None):
+        b = b200.DeviceBatch([n], [0.01])
+        if shape is not None:
+            b.set_shape(*shape)
+        b.set_state(0, d["x"], d["y"], d["z"], d["vx"], d["vy"], d["vz"], d["m"])
+        b.refresh()
+        return b
+
+    def step_seconds(b):
+        times = []
+        for _ in range(9):
+            start = time.perf_counter()
+            b.step(1e-4, 20, "vv")
+            times.append(time.perf_counter() - start)
+        return np.median(times)
+
+    tuned = batch()
+    shape, ms = tuned.autotune()
+    seconds = step_seconds(tuned)
+    assert ms > 0 and seconds < 1.08 * step_seconds(batch())
+    assert seconds < 1.08 * step_seconds(batch((256, 2, by_size, 8)))
+    # What tuning returns can be set by hand.
+    a, b = tuned.state(0), batch(shape)
+    b.step(1e-4, 180, "vv")
+    for k in ("x", "vx", "ax"):
+        assert np.array_equal(a[k], b.state(0)[k]), k
