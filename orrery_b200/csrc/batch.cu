@@ -296,6 +296,14 @@ uint64_t Batch::footprint(uint32_t n) {
     return static_cast<uint64_t>(ceil_div(n, kDirectTile)) * kDirectTile;
 }
 
+uint64_t Batch::device_bytes(uint32_t n) {
+    const uint32_t tiles = std::max(1u, ceil_div(n, kDirectTile));
+    const uint32_t chunks = ceil_div(tiles, kDefaultConfig.chunk_of(tiles));
+    const uint64_t bt = kDefaultConfig.targets_per_block();
+    const uint64_t slots = chunks > 1 ? static_cast<uint64_t>(ceil_div(n, bt)) * chunks : 0;
+    return footprint(n) * kBytesPerParticle + slots * 3 * bt * sizeof(double);
+}
+
 void Batch::init(uint64_t capacity, cudaStream_t stream) {
     // Slack past the arena for target tiles that run over (<= 1024).
     const uint64_t total = capacity + 1024;
@@ -479,10 +487,7 @@ std::vector<BatchItem> Batch::make_items(const BatchConfig &config,
     for (const uint32_t s : ids) {
         const Member &m = members_[s];
         const uint32_t tiles = ceil_div(m.count, kDirectTile);
-        const uint32_t wanted = config.chunk_tiles != kChunkBySize ? config.chunk_tiles
-                                : tiles <= 8u                      ? 2u
-                                                                   : 8u;
-        const uint32_t chunk = wanted == 0 ? tiles : std::min(wanted, tiles);
+        const uint32_t chunk = config.chunk_of(tiles);
         const uint32_t chunks = ceil_div(tiles, chunk);
         for (uint32_t t = 0; t < m.count; t += bt) {
             const uint32_t n_targets = std::min(bt, m.count - t);

@@ -58,6 +58,11 @@ struct BatchConfig {
     [[nodiscard]] uint32_t targets_per_block() const {
         return static_cast<uint32_t>(threads * targets_per_thread / groups);
     }
+    // Source tiles per item of a system of `tiles` tiles.
+    [[nodiscard]] uint32_t chunk_of(uint32_t tiles) const {
+        const uint32_t wanted = chunk_tiles != kChunkBySize ? chunk_tiles : tiles <= 8u ? 2u : 8u;
+        return wanted == 0 || wanted > tiles ? tiles : wanted;
+    }
 };
 
 // (threads, targets per thread, source groups) of the implemented batched
@@ -109,6 +114,9 @@ public:
     static uint64_t footprint(uint32_t n);
     // Device bytes per padded particle of the arena.
     static constexpr uint64_t kBytesPerParticle = 10 * 8 + 64;
+    // Device bytes that a system of n particles takes with the default shape: its
+    // part of the arena and the partial sums of its chunks.
+    static uint64_t device_bytes(uint32_t n);
 
     void set_state(uint32_t id, const double *x, const double *y, const double *z,
                    const double *vx, const double *vy, const double *vz, const double *m);
@@ -168,7 +176,8 @@ private:
     // Four targets per thread read half the shared memory per interaction that
     // two do: a Yoshida step of 128 systems of 256 to 16,384 particles 15.8 ->
     // 14.4 ms.
-    BatchConfig config_{256, 4, kChunkBySize, 8};
+    static constexpr BatchConfig kDefaultConfig{256, 4, kChunkBySize, 8};
+    BatchConfig config_ = kDefaultConfig;
     bool dirty_ = true;
     uint32_t item_count_ = 0;
     uint32_t group_count_ = 0;

@@ -62,13 +62,13 @@ double percentile(std::vector<double> v, double q) {
 }
 
 // Device bytes a tree job holds: state (80 B per particle), ordering, sorted
-// copy and leaf records (88 B per particle) and about 0.75 N + 1024 nodes at
-// 188 B (FP64 node 64, quadrupole 48, walk record 64, first particle 4, child
-// and arrival counts 8).
-uint64_t tree_job_bytes(uint64_t n) { return n * 80 + n * 88 + (n * 3 / 4 + 1024) * 188; }
+// copy and leaf records (80 B per particle, look-back words included) and about
+// 0.75 N + 1024 nodes at 220 B (FP64 node 64, quadrupole 48, walk record 64 and
+// its index 4, child slots 32, child masks and arrival counts 8).
+uint64_t tree_job_bytes(uint64_t n) { return n * 80 + n * 80 + (n * 3 / 4 + 1024) * 220; }
 
 uint64_t direct_job_bytes(uint64_t n) {
-    return Batch::footprint(static_cast<uint32_t>(n)) * Batch::kBytesPerParticle;
+    return Batch::device_bytes(static_cast<uint32_t>(n));
 }
 
 struct Job {

@@ -92,6 +92,29 @@ def test_budget_holds_jobs_back_until_memory_frees():
         s.close()
 
 
+# 144 bytes per particle of the arena (whole tiles of 512), and 24 per target
+# (whole groups of 128) and chunk of the sources: none up to 1,024 particles, two
+# tiles per chunk to 4,096, eight above.
+@pytest.mark.parametrize("n,chunks", [(700, 0), (1024, 0), (1025, 2), (3000, 3), (4096, 4),
+                                      (4097, 2), (20011, 5)])
+def test_a_direct_job_s_bytes_hold_its_partial_sums(n, chunks):
+    tiles, groups = -(-n // 512), -(-n // 128)
+    expected = 144 * 512 * tiles + 24 * 128 * groups * chunks
+    for budget, code in ((expected, None), (expected - 1, ob.ERROR_CAPACITY)):
+        s = ob.Server(hbm_budget_bytes=budget, fake=True)
+        try:
+            if code is None:
+                s.wait(s.submit(_state(n), steps=1, dt=1e-3, softening=0.01), timeout=60,
+                       outputs=False)
+                assert s.stats()["hbm_peak"] == expected
+            else:
+                with pytest.raises(ob.OrreryError) as err:
+                    s.submit(_state(n), steps=1, dt=1e-3, softening=0.01)
+                assert err.value.code == code
+        finally:
+            s.close()
+
+
 def test_a_job_that_never_fits_is_refused():
     s = ob.Server(hbm_budget_bytes=10_000_000, fake=True)
     try:
