@@ -575,14 +575,15 @@ __global__ void __launch_bounds__(OrderedShape<ForceTerm>::threads)
 // overlap, and added in index order. Each warp stages its own sources.
 constexpr uint32_t kAhead = 4;
 constexpr uint32_t kWideThreads = 64;
-// From here on one target per thread: with the terms formed by many warps,
-// and one target per thread, an evaluation took 242 and 482 us at 8,192
-// targets, 898 and 952 us at 16,384 (0.9 warps per SM sub-partition), 3.08 and
-// 2.66 ms at 32,768 (shared memory carries 48 bytes per pair there), 12.1 and
-// 9.9 ms at 65,536. The former single kernel (one target per thread, the
-// general root and division, 128-thread CTAs): 731 us at 4,096, 2.91 ms at
-// 16,384, 15.3 ms at 65,536.
-constexpr uint32_t kWideFrom = 16384;
+// From here on one target per thread: past two full waves of the other kernel's
+// CTAs (three of 32 targets per SM, 148 SMs). With the terms formed by many warps,
+// and one target per thread, an evaluation took 242 and 482 us at 8,192 targets,
+// 904 and 958 us at 16,384, 1.62 and 1.93 ms at 23,680, 2.31 ms both at 28,416, 2.82
+// and 2.44 ms at 30,000 (a third wave; shared memory carries 48 bytes per pair),
+// 12.1 and 10.0 ms at 65,536. The former single kernel (one target per thread, the
+// general root and division, 128-thread CTAs): 731 us at 4,096, 2.91 ms at 16,384,
+// 15.3 ms at 65,536.
+constexpr uint32_t kWideFrom = 2 * 3 * 148 * 32 + 1;
 
 __global__ void __launch_bounds__(kWideThreads)
     direct_f64_wide_kernel(const double *__restrict__ x, const double *__restrict__ y,

@@ -37,7 +37,7 @@ def test_fp64_is_bit_identical_to_reference(b200, golden_plummer):
         assert s.interaction_count().particle_particle == 2048 * 2047
 
 
-# 31-33: the edges of a chunk of sources; 16,384 and on: one target per thread.
+# 31-33: the edges of a chunk of sources; 28,417 and on: one target per thread.
 # The scales put squared distances below and above the range of the short
 # root and division; without softening the target's own argument is zero. (Below
 # that range, |d|^2 < 2^-895, the force's 1 / |d|^3 > 2^1342 overflows, in the
@@ -46,7 +46,8 @@ def test_fp64_is_bit_identical_to_reference(b200, golden_plummer):
                                          (33, 0.05, 1.0), (257, 0.0, 1e-140),
                                          (257, 0.0, 1e137), (4097, 0.01, 1.0),
                                          (16383, 0.01, 1.0), (16384, 0.01, 1.0),
-                                         (16415, 0.0, 1.0)])
+                                         (16415, 0.0, 1.0), (28416, 0.01, 1.0),
+                                         (28417, 0.0, 1.0), (28447, 0.01, 1.0)])
 def test_fp64_sums_are_bit_identical_at_every_size(b200, restatement, n, eps, scale):
     from orrery_b200 import initial_conditions as ic
     d = ic.plummer_sphere(n, seed=n)
