@@ -474,6 +474,13 @@ def run_reference(args, w):
     if rank != 0:
         barrier(dist)
         return
+    import oracle
+
+    if not oracle.Reference.available():
+        print(json.dumps({"impl": "reference", "unavailable": "the reference library "
+                          "(oracle/_ref) is not built: its sources are not here"}), flush=True)
+        barrier(dist)
+        return
     steps = max(1, args.steps)
     if w["kind"] == "serving":
         base = cpu_baseline_serving(w, budget_s=min(60.0, 10.0 * steps))

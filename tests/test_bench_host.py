@@ -3,10 +3,13 @@ seeded and has the stated mix, job inputs are valid systems, and the traffic
 and roofline constants scale with the work."""
 from __future__ import annotations
 
+import json
 import os
 import sys
+from types import SimpleNamespace
 
 import numpy as np
+import pytest
 
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 sys.path.insert(0, ROOT)
@@ -44,3 +47,15 @@ def test_traffic_scales_with_the_work():
     assert t[("walk", "fp32")](2_000_000) == 4 * t[("walk", "fp32")](500_000)
     assert t[("direct", "split")](262_144) > t[("direct", "fp32")](262_144)
     assert abs(t[("batch", "split")](1.7416705824e10) - 258.9e6) < 1.0
+
+
+@pytest.mark.parametrize("workload", sorted(bench.WORKLOADS))
+def test_reference_arm_without_the_reference_says_so_and_times_nothing(monkeypatch, capsys,
+                                                                       workload):
+    import oracle
+    monkeypatch.setattr(oracle.Reference, "available", staticmethod(lambda: False))
+    monkeypatch.setattr(oracle, "Restatement", None)  # a stand-in would be no reference
+    args = SimpleNamespace(gpus=1, steps=1, warmup=3, workload=workload)
+    bench.run_reference(args, bench.WORKLOADS[workload])
+    line = json.loads(capsys.readouterr().out.strip())
+    assert set(line) == {"impl", "unavailable"} and line["impl"] == "reference"
