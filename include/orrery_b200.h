@@ -562,9 +562,9 @@ int ob_test_tree_timeout(ob_solver *solver, uint32_t stage, uint32_t poll_limit)
 /* Bounds the FP32 tree walk's traversal stack of `solver` to `cap` (at most
  * 256) entries (0 restores the full stack) from its next evaluation on. A group
  * of targets whose stack fills discards its partial sums and finishes with the
- * per-target union walk (the fallback a valid tree rarely needs); a small cap forces it,
- * so tests can hold that path to the oracle. OB_ERROR_UNSUPPORTED for direct
- * or FP64 solvers. No reference counterpart. */
+ * per-target union walk (the fallback a valid tree rarely needs); a small cap
+ * forces it, so tests can hold that path to the oracle. OB_ERROR_UNSUPPORTED for
+ * direct or FP64 solvers. No reference counterpart. */
 int ob_test_set_walk_stack_cap(ob_solver *solver, uint32_t cap);
 
 /* Arms the next fused launch of `system` (ob_system_set_fused_steps) for a

@@ -13,8 +13,9 @@
 // of thousands of targets and waits on each term's dependent chain (4,096
 // targets: 32 CTAs, 734 us; potential energy of 32,768: 5.7 ms). Here the chain
 // per source is one FP64 addition: 4,096 targets 77 us, potential 1.0 ms. What
-// bounds it: at one CTA per SM the latency of a chunk (the FP64 pipe is 36 %
-// busy), at several the shared memory that carries the terms.
+// bounds it: at one CTA per SM the latency of a chunk (4,096 targets, 16 term
+// warps: the FP64 pipe is 42 % busy, issue slots 58 %), at several the shared
+// memory that carries the terms.
 #pragma once
 
 #include <cstdint>

@@ -22,9 +22,9 @@
 //      shared memory by one bulk copy, once the ready words of the CTAs that
 //      wrote it have reached this substep (no grid-wide barrier: a warp waits,
 //      on its own mbarrier, only for the slice it sums; with one mbarrier for
-//      the whole CTA a 64-particle step took 3.0 us,
-//      now 2.4, a 1,000-particle one 5.5, now 4.7, a 5,500-particle one 28.4,
-//      now 25.0; 4,096, bound by the pair loop's FP32 pipe, 11.9 and 11.8);
+//      the whole CTA a 64-particle step took 3.0 us, now 2.4, a 1,000-particle
+//      one 5.5, now 4.7, a 5,500-particle one 28.4, now 25.0; at 4,096, one CTA
+//      per SM, it makes no difference: 11.8 us);
 //   C. the CTA evaluates its targets' accelerations: FP32 pair arithmetic
 //      two sources per packed FP32x2 instruction, each warp's slice summed
 //      in FP32, the W slices added in FP64 in slice order by warp 0.
@@ -38,9 +38,9 @@
 // far, `epoch`, and clears the words together with it); waits are bounded
 // (kSpinLimit polls, or fewer where a test asks, then the timeout bit of the
 // status word, and every CTA stops after the substep it is in), and the
-// launch is cooperative, so every CTA is resident. The pair arithmetic is that of the FP32 direct kernel
-// (positions rounded to FP32, softened, FP32 sums per slice, FP64 across
-// slices); with softening the target's own entry adds exactly zero unless
+// launch is cooperative, so every CTA is resident. The pair arithmetic is that
+// of the FP32 direct kernel (positions rounded to FP32, softened, FP32 sums per
+// slice, FP64 across slices); with softening the target's own entry adds exactly zero unless
 // m / eps^3 of the target overflows FP32, in which case the warp skips it
 // explicitly.
 #include <algorithm>

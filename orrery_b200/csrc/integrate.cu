@@ -131,7 +131,8 @@ __global__ void kinetic_terms_kernel(const double *__restrict__ vx, const double
 // ones fill in behind them.
 struct PotentialTerm {
     static constexpr int components = 1;
-    static constexpr int warps = 8; // 65,536 rows: 4.1 ms with the host's part, with 16 warps 5.2 ms
+    // 65,536 rows: 4.1 ms with the host's part, with 16 warps 5.2 ms.
+    static constexpr int warps = 8;
     static __device__ __forceinline__ void form(double m, double inv, double, double, double,
                                                 double (&term)[1]) {
         term[0] = __dmul_rn(m, inv);

@@ -13,8 +13,9 @@
 // size, allocated by the CUDA runtime when the library is loaded on a device
 // and held by every device that loads it until the process exits.
 //
-// The kernels are the ones the tree solver uses (sort.cu); only where their
-// scratch comes from differs.
+// The device code is the one the tree solver's ordering uses (sort.cu), launched
+// phase by phase instead of in one cooperative kernel; where the scratch comes from
+// differs too.
 #include <cstdint>
 #include <mutex>
 

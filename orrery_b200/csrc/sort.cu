@@ -11,11 +11,16 @@
 //     (code, index) ordering (include/orrery/solvers/morton.hpp:155-175).
 //
 // The sort: one histogram pass (fused into encoding) computes all eight digit
-// histograms; then each of the eight passes is a single kernel in which a CTA
-// takes the next tile in launch order (ticket counter), ranks its keys stably
-// with warp match operations, publishes its per-digit counts, resolves its
-// global offsets by decoupled look-back over earlier tiles (every wait bounded)
-// and scatters through shared memory so the global writes are contiguous runs.
+// histograms; in each of the eight passes a CTA takes a tile, ranks its keys
+// stably with warp match operations, publishes its per-digit counts, resolves
+// its global offsets by decoupled look-back over earlier tiles (every wait
+// bounded) and scatters through shared memory so the global writes are
+// contiguous runs.
+//
+// Two routes launch these pieces. The tree's (order_kernel) is one cooperative
+// launch for all of it, with a grid barrier between phases and tiles given to
+// the CTAs in ascending order. ob_morton_order_noalloc launches each phase by
+// itself; there a CTA takes the next tile in launch order from a ticket counter.
 #include <algorithm>
 #include <atomic>
 

@@ -795,8 +795,8 @@ void TreePipeline::evaluate(uint32_t n, const double *x, const double *y, const 
     const WalkNodes walk{records, records + node_capacity_, records + 2ull * node_capacity_,
                          records + 3ull * node_capacity_, walk_index_.data()};
     check(launch_layout(codes, n, cap, offsets, scan_partials_.data(), node_capacity_,
-                        nodes_.data(), child_mask, child_slots, perms[0], meta_.data(), barriers + 1,
-                        status, stream, silent, polls),
+                        nodes_.data(), child_mask, child_slots, perms[0], meta_.data(),
+                        barriers + 1, status, stream, silent, polls),
           "node layout");
     check(launch_moments(sorted_.data(), codes, n, nodes_.data(),
                          params_.quadrupole ? quads_.data() : nullptr, walk, child_mask,

@@ -118,8 +118,8 @@ public:
     // Raises the node capacity used from the next evaluation on.
     void grow_nodes(uint32_t at_least);
 
-    // Bounds the walk's per-warp traversal stack (0 = its full capacity) from
-    // the next evaluation on; a warp whose stack fills finishes with the
+    // Bounds the walk's traversal stack (0 = its full capacity) from the next
+    // evaluation on; a group of targets whose stack fills finishes with the
     // per-target union walk. For tests of that fallback.
     void set_walk_stack_cap(uint32_t cap) noexcept { walk_stack_cap_ = cap; }
 

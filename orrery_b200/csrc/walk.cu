@@ -18,8 +18,8 @@
 // word and a node's children are all met in the round after it. (With one
 // stack item per node that pushed its next sibling, a path down the tree cost
 // one round per sibling: 104 us for 1,000 particles, bound by that chain.)
-// Each lane classifies its node against the
-// bounding box of the group's targets from the node's compact record: the
+// Each lane classifies its node against the bounding box of the group's targets
+// from the node's compact record: the
 // per-axis distances from the centre of mass to the nearest and farthest box
 // faces are formed from FP32 hi + lo parts (so each is accurate to a few ulps
 // of itself), and with a 4e-6 relative margin on the acceptance radius
@@ -71,14 +71,15 @@
 // kStatusInvalid and is skipped.
 //
 // Bound by FP32 issue and the latency between dependent steps: at 200,000
-// particles (quadrupoles, two warps per group) the FMA pipe is 48 % busy and
-// 60 % of issue slots are used. Walk times, before (one warp per group, one
-// stack item per node) and after: 10,000 Plummer particles without quadrupoles
-// 367 -> 119 us; 100,000 collision particles 752 -> 672 us; 200,000 1.41 -> 1.33
-// ms; 2,000,000 14.89 -> 14.72 ms. Relative error against the FP64 walk (2-norm):
-// 10,000 8.1e-8 -> 5.3e-8, 200,000 3.89e-8 -> 3.78e-8, 2,000,000 3.73e-8 ->
-// 3.70e-8 (flush_cells says how the cells are summed). Groups of 64 targets (two
-// per lane) halve the traversal but measured no faster at any size.
+// particles (quadrupoles, two warps per group) the FMA pipe is 48 % busy and 61 %
+// of issue slots are used, at 500,000 (one warp per group) 57 % and 67 %. Walk
+// times, before (one warp per group, one stack item per node) and after: 10,000
+// Plummer particles without quadrupoles 367 -> 119 us; 100,000 collision particles
+// 752 -> 672 us; 200,000 1.41 -> 1.33 ms; 2,000,000 14.89 -> 14.72 ms. Relative
+// error against the FP64 walk (2-norm): 10,000 8.1e-8 -> 5.3e-8, 200,000 3.89e-8 ->
+// 3.78e-8, 2,000,000 3.73e-8 -> 3.70e-8 (flush_cells says how the cells are summed).
+// Groups of 64 targets (two per lane) halve the traversal but measured no faster at
+// any size.
 #include <algorithm>
 #include <atomic>
 
@@ -569,7 +570,8 @@ __device__ __forceinline__ void flush_leaves(WarpSpace &ws, uint32_t count,
 }
 
 // 28 warps per SM at 72 registers: with 32 at 64 the quadrupole walk spills
-// (2M 15.1 ms against 14.4), 24 at 80 hide less latency (15.0 ms).
+// (2M 15.1 ms against 14.4, both with cells in blocks of sixteen), 24 at 80 hide
+// less latency (15.0 ms).
 template <bool QUAD, int W>
 __global__ void __launch_bounds__(Shape<W>::threads, 896 / Shape<W>::threads)
     walk_kernel(const DeviceNode *__restrict__ nodes,

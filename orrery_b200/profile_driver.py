@@ -2,6 +2,7 @@
 
     python -m orrery_b200.profile_driver tree N      # Barnes-Hut evaluations of the
                                                      # two-disc collision of N particles
+    python -m orrery_b200.profile_driver fp64 N      # FP64 direct solver, Plummer sphere of N
     python -m orrery_b200.profile_driver pack        # FP32 direct solver, Plummer 262,144
     python -m orrery_b200.profile_driver batch       # 64 clusters (3 above 8192 particles)
                                                      # in chunked batched items
@@ -27,6 +28,15 @@ def tree(n: int) -> None:
 
     d = ic.galaxy_collision(n, softening=0.02, seed=20260811)
     solver = B200TreeSolver(0.02, 0.5, 32, True)
+    for _ in range(4):
+        solver.evaluate((d["x"], d["y"], d["z"]), d["m"])
+
+
+def fp64(n: int) -> None:
+    from . import B200DirectSolver
+
+    d = ic.plummer_sphere(n, seed=8)
+    solver = B200DirectSolver(0.01, "fp64")
     for _ in range(4):
         solver.evaluate((d["x"], d["y"], d["z"]), d["m"])
 
@@ -84,8 +94,8 @@ def main(argv: list[str]) -> None:
 
     load_library()
     what = argv[1] if len(argv) > 1 else ""
-    if what == "tree":
-        tree(int(argv[2]))
+    if what in ("tree", "fp64"):
+        {"tree": tree, "fp64": fp64}[what](int(argv[2]))
     elif what in ("pack", "batch", "rk4", "fused"):
         {"pack": pack, "batch": batch, "rk4": rk4, "fused": fused}[what]()
     else:

@@ -124,6 +124,32 @@ def test_a_full_traversal_stack_falls_back_to_the_union_walk(b200, restatement, 
                                                         counts.particle_cell)
 
 
+# 4, 2 and 1 warps per group of 32 targets (the test above: 8), and monopoles.
+@pytest.mark.parametrize("n,quad", [(70_000, True), (70_000, False), (140_000, True),
+                                    (140_000, False), (262_145, True), (262_145, False),
+                                    (20_000, False)])
+def test_every_number_of_warps_falls_back_to_the_union_walk(b200, restatement, n, quad):
+    from orrery_b200 import initial_conditions as ic
+    lib = b200.load_library()
+    lib.ob_test_set_walk_stack_cap.argtypes = [C.c_void_p, C.c_uint32]
+    lib.ob_test_set_walk_stack_cap.restype = C.c_int
+    d = ic.galaxy_collision(n, softening=0.02, seed=n)
+    x, y, z, m = d["x"], d["y"], d["z"], d["m"]
+    a_ref, counts = restatement.barnes_hut(x, y, z, m, 0.02, 1.0, 24, quad)
+    solver = b200.B200TreeSolver(0.02, 1.0, 24, quad)
+    whole = solver.evaluate((x, y, z), m)
+    for cap in (2, 40):  # every group falls back; some do
+        assert lib.ob_test_set_walk_stack_cap(solver._handle, cap) == b200.OK
+        solver.reset_interaction_count()
+        a = solver.evaluate((x, y, z), m)
+        c = solver.interaction_count()
+        assert (c.particle_particle, c.particle_cell) == (counts.particle_particle,
+                                                          counts.particle_cell)
+        err = np.linalg.norm(a - a_ref, axis=1) / np.linalg.norm(a_ref, axis=1)
+        assert err.max() < 1e-4 and np.sqrt(np.mean(err ** 2)) < 1e-5
+        assert not np.array_equal(a, whole)  # another order of sums: it did fall back
+
+
 def test_the_stack_cap_is_refused_where_it_does_not_apply(b200):
     lib = b200.load_library()
     lib.ob_test_set_walk_stack_cap.argtypes = [C.c_void_p, C.c_uint32]
