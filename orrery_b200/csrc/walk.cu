@@ -74,8 +74,8 @@
 // particles (quadrupoles, two warps per group) the FMA pipe is 48 % busy and 61 %
 // of issue slots are used, at 500,000 (one warp per group) 57 % and 67 %. Walk
 // times, before (one warp per group, one stack item per node) and after: 10,000
-// Plummer particles without quadrupoles 367 -> 119 us; 100,000 collision particles
-// 752 -> 672 us; 200,000 1.41 -> 1.33 ms; 2,000,000 14.89 -> 14.72 ms. Relative
+// Plummer particles without quadrupoles 367 -> 118 us; 100,000 collision particles
+// 752 -> 660 us; 200,000 1.41 -> 1.30 ms; 2,000,000 14.89 -> 14.43 ms. Relative
 // error against the FP64 walk (2-norm): 10,000 8.1e-8 -> 5.3e-8, 200,000 3.89e-8 ->
 // 3.78e-8, 2,000,000 3.73e-8 -> 3.70e-8 (flush_cells says how the cells are summed).
 // Groups of 64 targets (two per lane) halve the traversal but measured no faster at
@@ -420,7 +420,8 @@ __device__ __forceinline__ void cell_pair(const WarpSpace &ws, uint32_t p, float
 // are summed in blocks of eight: 2-norm error against the FP64 walk at 200,000
 // and 2,000,000 particles (collision) 3.78e-8 and 3.70e-8, in blocks of sixteen
 // 3.91e-8 and 3.85e-8, one chain over cells in pre-order 3.89e-8 and 3.73e-8
-// (walk 14.7, 14.5 and 14.9 ms at 2,000,000). Monopole cells, whose terms are
+// (walk 14.4, 14.5 and 14.9 ms at 2,000,000; whole blocks are written out, in one
+// loop with the last one 14.7 ms). Monopole cells, whose terms are
 // shorter, go to two chains by turns, which meet in FP64: 1,000,000 Plummer
 // particles 3.61e-8 and 4.62 ms, in blocks of eight 3.74e-8 and 4.79 ms, of
 // sixteen 3.77e-8 and 4.70 ms, one pre-order chain 3.65e-8 and 4.70 ms.
@@ -439,10 +440,21 @@ __device__ __forceinline__ void flush_cells(WarpSpace &ws, uint32_t count, float
     __syncwarp();
     if constexpr (QUAD) {
         float2 sx = f2(0.0f, 0.0f), sy = sx, sz = sx;
-        for (uint32_t from = 0; from < count; from += kCellBlock) {
-            const uint32_t to = min(from + kCellBlock, count);
+        const uint32_t whole = count & ~(kCellBlock - 1u); // cells of whole blocks
+#pragma unroll 1
+        for (uint32_t from = 0; from < whole; from += kCellBlock) {
             float2 bx = f2(0.0f, 0.0f), by = bx, bz = bx;
-            for (uint32_t j = from; j < to; j += 2) {
+#pragma unroll
+            for (uint32_t p = 0; p < kCellBlock / 2u; ++p) {
+                cell_pair<true>(ws, (from >> 1) + p, ntx, nty, ntz, eps2, lane_bit, bx, by, bz);
+            }
+            sx = __fadd2_rn(sx, bx);
+            sy = __fadd2_rn(sy, by);
+            sz = __fadd2_rn(sz, bz);
+        }
+        if (whole < count) {
+            float2 bx = f2(0.0f, 0.0f), by = bx, bz = bx;
+            for (uint32_t j = whole; j < count; j += 2) {
                 cell_pair<true>(ws, j >> 1, ntx, nty, ntz, eps2, lane_bit, bx, by, bz);
             }
             sx = __fadd2_rn(sx, bx);
