@@ -331,6 +331,8 @@ def cpu_baseline_batch(w, sizes, radii, systems, budget_s=15.0):
     is spent; the rate over the systems done stands for the batch."""
     import oracle
 
+    if not oracle.Reference.available():
+        return {"unavailable": "the reference library (oracle/_ref) is not built"}
     ref = oracle.Reference()
     threads = ref.worker_count()
     done_pairs, spent, count = 0, 0.0, 0

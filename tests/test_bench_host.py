@@ -59,3 +59,10 @@ def test_reference_arm_without_the_reference_says_so_and_times_nothing(monkeypat
     bench.run_reference(args, bench.WORKLOADS[workload])
     line = json.loads(capsys.readouterr().out.strip())
     assert set(line) == {"impl", "unavailable"} and line["impl"] == "reference"
+
+
+def test_a_batch_s_baseline_without_the_reference_does_not_raise(monkeypatch):
+    import oracle
+    monkeypatch.setattr(oracle.Reference, "available", staticmethod(lambda: False))
+    w = bench.WORKLOADS["batched-512"]
+    assert set(bench.cpu_baseline_batch(w, [256], [1.0], [{}])) == {"unavailable"}
